@@ -47,6 +47,32 @@ def main():
         h, l = dd(mp.atan(mp.mpf(j) / 64))
         out.append(f"    {{{fmt(h)}, {fmt(l)}}},  // j = {j}")
     out.append("};")
+    # quick log: mantissas z in [kLogQOff, 2 kLogQOff) by the top 7 bits above the offset; rc is a reciprocal of the
+    # interval short enough (8 fraction bits above 1, 7 below) that z rc - 1 is exact in one fma, 1 on the two
+    # intervals beside z = 1; -log rc with its high part a multiple of 2^-42, so that k kLn2Hi + hi is exact
+    out.append("// {rc, hi, lo, 0} of the 128 mantissa intervals: |z rc - 1| < 2^-7, hi + lo = -log rc, hi a multiple of 2^-42")
+    out.append("constexpr unsigned kLogQOff = 0x3fe6a000u;  // high word of the first interval's start")
+    out.append("SC_DDM_TABLE double kLogQ[128][4] = {")
+    for i in range(128):
+        def z(hw):
+            e = (hw >> 20) - 1023
+            return mp.ldexp(1 + mp.mpf(hw & 0xfffff) / 2 ** 20, e)
+        a, b = z(0x3fe6a000 + i * 0x2000), z(0x3fe6a000 + (i + 1) * 0x2000)
+        q = 128 if a < 1 else 256
+        rc = mp.mpf(1) if i in (74, 75) else mp.nint(q / ((a + b) / 2)) / q
+        assert max(abs(a * rc - 1), abs(b * rc - 1)) <= mp.mpf(2) ** -7
+        t = -mp.log(rc)
+        th = mp.nint(mp.ldexp(t, 42)) / mp.mpf(2) ** 42
+        out.append(f"    {{{fmt(float(rc))}, {fmt(float(th))}, {fmt(float(t - th))}, 0.0}},")
+    out.append("};")
+    out.append("// row j: atan(j / 128); row 129 + j: pi / 2 - atan(j / 128), j = 0 .. 128: {hi, lo}")
+    out.append("SC_DDM_TABLE double kAtanQ[258][2] = {")
+    for inv in (0, 1):
+        for j in range(129):
+            t = mp.atan(mp.mpf(j) / 128)
+            h, l = dd(mp.pi / 2 - t if inv else t)
+            out.append(f"    {{{fmt(h)}, {fmt(l)}}},")
+    out.append("};")
     # ln2 split so that k * hi is exact for |k| < 2^11: hi keeps 42 significant bits
     m, e = mp.frexp(mp.log(2))
     hi = mp.ldexp(mp.floor(mp.ldexp(m, 42)), e - 42)

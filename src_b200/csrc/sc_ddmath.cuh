@@ -186,151 +186,137 @@ SC_DDM_HD double atan_dd_full(double x) {
 
 // ---------------------------------------------------------------- quick phase
 // Ziv's strategy (as in CRlibm, Daramy-Loirat et al.): a cheaper evaluation
-// whose result hi + lo carries a relative error below kQuickEps; when that
-// error cannot move the value across a rounding boundary, hi is the
-// correctly rounded result, otherwise the full double-double evaluation
-// above decides.  log and atan of a double other than log 1, atan 0 are
-// transcendental, never exactly halfway between two doubles.  The quick
-// phase accepts only values at least 2^-10 ulp from a boundary, where the
-// full evaluation is correctly rounded too, so both phases give the same
-// bits.
+// hi + lo with a proven error bound E; when hi + (lo - E) and hi + (lo + E)
+// round to the same double, that double is the correctly rounded result,
+// otherwise the full double-double evaluation above decides.  log and atan of
+// a double other than log 1, atan 0 are transcendental, never exactly halfway
+// between two doubles, and the accepted values keep a distance from the
+// boundaries at which the full evaluation is correctly rounded too, so both
+// phases give the same bits.
 //
-// Error budget of both quick phases, relative to the result v: the
-// argument reduction t = th + tl is exact to 2^-103; the polynomial tail
-// above the last exactly summed term is below 2^-14.5 |v| and is evaluated
-// with a relative error under 2^-51; the low-order words (at most about
-// ten, each below 2^-14.5 |v|) are added in double with at most 2^-53 of
-// their partial sums per addition.  Together about 2^-65 |v| at worst (the
-// largest error seen against quad precision, over 2e7 arguments spread over
-// every table interval, is 2^-65.5); the test allows 2^-63.
-constexpr double kQuickEps = 0x1p-63;
+// The Green's function evaluates three of each per mesh point and is bound by
+// the FP64 pipe, so both reductions are chosen for few operations: exact
+// arguments from one fused multiply-add, low parts added in double, one
+// rounding test in place of a renormalisation.  About 23 FP64 operations for
+// log and 33 for atan (the first form, a 64-interval reduction with TwoSums
+// throughout, took about 60 and 80): the Green's-function phase 175 -> 134 us
+// at 128^3 and 41.6 -> 35.4 us at 64^3, the same bits.
+struct hilo {
+    double hi, lo;
+};
 
-// RN(hi + lo + d) == hi for every |d| <= eps |hi|, with |lo| <= ulp(hi) / 2
-// and hi normal; powers of two (a smaller ulp below) are left to the full
-// evaluation.
-SC_DDM_HD bool rounds_to_hi(double hi, double lo, double eps) {
+SC_DDM_HD uint64_t bits_of(double x) {
     uint64_t b;
-    memcpy(&b, &hi, sizeof b);
-    if ((b & 0x000fffffffffffffull) == 0) return false;
-    b &= 0x7ff0000000000000ull;
-    if (b < 0x07b0000000000000ull) return false;  // |hi| < 2^-900: left to the full evaluation
-    double half_ulp;
-    memcpy(&half_ulp, &b, sizeof half_ulp);
-    half_ulp *= 0x1p-53;
-    return fabs(lo) + eps * fabs(hi) < half_ulp;
+    memcpy(&b, &x, sizeof b);
+    return b;
+}
+SC_DDM_HD double double_of(uint64_t b) {
+    double x;
+    memcpy(&x, &b, sizeof x);
+    return x;
 }
 
-// Quick log: the reduction of log_dd_full; log1p t = t - t^2/2 + t^3 q(t)
-// with t^2 exact (TwoProd) and t^3 q(t) in double; k log2 + log c + th -
-// th^2/2 by exact TwoSums, the rest as one double.
+// log x = k log 2 - log rc + log1p r for finite normal x: z = x 2^-k in
+// [0.707, 1.414), rc a short reciprocal of z's interval (kLogQ), r = z rc - 1
+// exact, |r| <= 2^-7.  k log 2 (high part) - log rc (high part) is exact
+// (both multiples of 2^-42); log1p r - r = r^2 (-1/2 + r/3 - ... + r^7/9) in
+// double.  exact: the sum s + r is an exact Fast2Sum (|s| >= 2^-7 or s == 0).
+// Error of hi + lo, where exact holds: the truncation of log1p below 2^-73,
+// the polynomial r^2 (...) < 2^-15 with at most 1.6 2^-53 of it, two
+// additions to lo (|lo| < 2^-14.9) 2^-68 each: together below 2^-66.3 (the
+// largest seen over 2e7 arguments is 2^-67.5).
+constexpr double kLogQuickErr = 0x1p-64;
+SC_DDM_HD hilo log_hilo(double x, bool& exact) {
+    const uint64_t b = bits_of(x);
+    const uint32_t h = (uint32_t)(b >> 32);
+    const uint32_t t = h - kLogQOff;
+    const int k = (int32_t)t >> 20;
+    const int i = (int)(t >> 13) & 127;
+    const double z = double_of(((uint64_t)(h - (t & 0xfff00000u)) << 32) | (uint32_t)b);
+    const double rc = kLogQ[i][0], th = kLogQ[i][1], tl = kLogQ[i][2];
+    const double r = fma(z, rc, -1.0);
+    double p = fma(r, 1.0 / 9.0, -1.0 / 8.0);
+    p = fma(r, p, 1.0 / 7.0);
+    p = fma(r, p, -1.0 / 6.0);
+    p = fma(r, p, 1.0 / 5.0);
+    p = fma(r, p, -1.0 / 4.0);
+    p = fma(r, p, 1.0 / 3.0);
+    p = fma(r, p, -0.5);
+    // k as a double: 2^52 + 2^31 + k has k + 2^31 in its low word (no conversion)
+    const double kd = double_of((uint64_t)0x43300000u << 32 | ((uint32_t)k ^ 0x80000000u)) - (0x1p52 + 0x1p31);
+    const double s = fma(kd, kLn2Hi, th);
+    exact = ((uint32_t)(bits_of(s) >> 32) & 0x7fffffffu) >= 0x3f800000u || s == 0.0;
+    const double hi = s + r;
+    double lo = fma(kd, kLn2Lo, tl);
+    lo = fma(r * r, p, lo);
+    lo += r - (hi - s);
+    return hilo{hi, lo};
+}
+
+// Quick log: false where the rounding is undecided.
 SC_DDM_HD bool log_quick(double x, double& out) {
-    uint64_t bits;
-    memcpy(&bits, &x, sizeof bits);
-    int k = (int)(bits >> 52) - 1023;
-    bits = (bits & 0x000fffffffffffffull) | 0x3ff0000000000000ull;
-    double m;
-    memcpy(&m, &bits, sizeof m);
-    if (m > 1.4142135623730951) {
-        m = m * 0.5;
-        k += 1;
-    }
-    const int j = (int)rint(m * 64.0);
-    const double c = (double)j / 64.0;
-    const double u = m - c;
-    const double rc = kLogRcp[j - kLogJ0];
-    const double th = u * rc;
-    const double tl = fma(-th, c, u) * rc;  // |t| < 2^-6.49
-    // q(t) = 1/3 - t/4 + t^2/5 - ... + t^8/11 (terms to t^11 of log1p)
-    double q = fma(th, 1.0 / 11.0, -1.0 / 10.0);
-    q = fma(th, q, 1.0 / 9.0);
-    q = fma(th, q, -1.0 / 8.0);
-    q = fma(th, q, 1.0 / 7.0);
-    q = fma(th, q, -1.0 / 6.0);
-    q = fma(th, q, 1.0 / 5.0);
-    q = fma(th, q, -1.0 / 4.0);
-    q = fma(th, q, 1.0 / 3.0);
-    const double p = th * th, pe = fma(th, th, -p);
-    const double cubic = (p * th) * q;
-    const double kd = (double)k;
-    const dd s1 = two_sum(kd * kLn2Hi, kLogTab[j - kLogJ0][0]);
-    const dd s2 = two_sum(s1.hi, th);
-    const dd s3 = two_sum(s2.hi, -0.5 * p);
-    double lo = -(th * tl) - 0.5 * pe;
-    lo += tl;
-    lo += kLogTab[j - kLogJ0][1];
-    lo += kd * kLn2Lo;
-    lo += s1.lo + s2.lo + s3.lo;
-    lo += cubic;
-    const dd r = fast_two_sum(s3.hi, lo);
-    if (!rounds_to_hi(r.hi, r.lo, kQuickEps)) return false;
-    out = r.hi;
-    return true;
+    bool exact;
+    const hilo v = log_hilo(x, exact);
+    out = v.hi + (v.lo + kLogQuickErr);
+    return exact && out == v.hi + (v.lo - kLogQuickErr);
 }
 
-// Reciprocal of d in [1, 2^31] to about 2^-52: the float reciprocal and two
-// Newton steps.
+// Reciprocal of d in [1, 2^31] to about 2^-52: an approximation to 2^-20 and
+// one step of third order.
 SC_DDM_HD double rcp_approx(double d) {
-    double r = (double)(1.0f / (float)d);
-    r = fma(r, fma(-d, r, 1.0), r);
-    r = fma(r, fma(-d, r, 1.0), r);
-    return r;
+    double r;
+#ifdef __CUDA_ARCH__
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+#else
+    r = (double)(1.0f / (float)d);
+#endif
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 
-// Quick atan for 2^-30 <= |x| <= 2^30: the reduction of atan_dd_full with
-// t = num / den to 2^-103 from one approximate reciprocal and the exact
-// residual, atan t = t + t^3 p(t^2) in double, atan c + th by TwoSum (and
-// pi/2 - that for |x| > 1).
-SC_DDM_HD bool atan_quick(double x, double& out) {
-    const double a = fabs(x);
+// atan a for 2^-30 <= a <= 2^30: c = j/128 near a (a <= 1) or near 1/a;
+//   a <= 1: atan a = atan c + atan t,        t = (a - c) / (1 + a c)
+//   a >  1: atan a = (pi/2 - atan c) + atan t, t = (a c - 1) / (a + c)
+// with |t| < 1.01 2^-8.  The numerator is exact in one fused multiply-add (c
+// has 8 bits, the difference cancels at least as many), the denominator is
+// dh + dl exactly, and t = th + tl to 2^-100 from the residual; atan t - t =
+// t^3 (-1/3 + t^2/5 - t^4 (1/7 - d)) in double, d = 0.92 of the next term's
+// t^2/9 at |t| = 2^-8, which leaves a truncation below 2^-69 t.  Error of
+// hi + lo relative to hi: below 2^-67.5 (largest for c = 0, where the tail
+// t^3/3 < 2^-17.5 t carries at most 3 2^-53 of itself; for c >= 1/128 the
+// tail is below 2^-18.5 hi; the largest seen over 2e7 arguments is 2^-67.8).
+constexpr double kAtanQuickEps = 0x1p-66;
+SC_DDM_HD hilo atan_hilo(double a) {
     const bool inv = a > 1.0;
-    // j = round(64 s), s = min(a, 1/a); a float 1/a may pick the neighbour
-    // of round(64/a), which keeps |t| below 2^-6.99
-    const int j = inv ? (int)rintf(64.0f / (float)a) : (int)rint(a * 64.0);
-    const double c = (double)j / 64.0;
-    double nh, nl, dh, dl;
-    if (inv) {
-        // 1 - a c may cancel to far below a c's low word: renormalise
-        const dd ac = two_prod(a, c);
-        const dd n = two_sum(1.0, -ac.hi);
-        const dd nn = two_sum(n.hi, n.lo - ac.lo);
-        nh = nn.hi;
-        nl = nn.lo;
-        const dd d = two_sum(a, c);
-        dh = d.hi;
-        dl = d.lo;
-    } else {
-        nh = a - c;  // exact (Sterbenz, or c = 0)
-        nl = 0.0;
-        const dd ac = two_prod(a, c);
-        const dd d = two_sum(1.0, ac.hi);
-        dh = d.hi;
-        dl = d.lo + ac.lo;
-    }
+    const float f = (float)a;
+    const int j = (int)rintf(inv ? 128.0f / f : 128.0f * f);
+    const int row = inv ? j + 129 : j;
+    const double th0 = kAtanQ[row][0], tl0 = kAtanQ[row][1];
+    // j / 128: 2^45 + j / 128 has j in its low word
+    const double c = double_of((uint64_t)0x42c00000u << 32 | (uint32_t)j) - 0x1p45;
+    const double u = inv ? a : 1.0, w = inv ? 1.0 : a;
+    const double num = inv ? fma(a, c, -1.0) : a - c;
+    const double dh = fma(w, c, u);
+    const double dl = fma(w, c, u - dh);
     const double rd = rcp_approx(dh);
-    const double th = nh * rd;
-    const double res = fma(-th, dh, nh) + (nl - th * dl);
-    const double tl = res * rd;
-    // atan t - t = t^3 (-1/3 + t^2/5 - t^4/7 + t^6/9 - t^8/11)
-    const double h2 = th * th;
-    double pq = fma(h2, -1.0 / 11.0, 1.0 / 9.0);
-    pq = fma(h2, pq, -1.0 / 7.0);
-    pq = fma(h2, pq, 1.0 / 5.0);
-    pq = fma(h2, pq, -1.0 / 3.0);
-    const double tail = (h2 * th) * pq;
-    const dd s1 = two_sum(kAtanTab[j][0], th);
-    double lo = tl + tail;
-    lo += kAtanTab[j][1];
-    lo += s1.lo;
-    double hi = s1.hi;
-    if (inv) {
-        const dd s2 = two_sum(kPiHalfHi, -hi);
-        lo = (kPiHalfLo - lo) + s2.lo;
-        hi = s2.hi;
-    }
-    const dd r = fast_two_sum(hi, lo);
-    if (!rounds_to_hi(r.hi, r.lo, kQuickEps)) return false;
-    out = x < 0.0 ? -r.hi : r.hi;
-    return true;
+    const double t = num * rd;
+    const double tl = fma(-t, dl, fma(-t, dh, num)) * rd;
+    const double t2 = t * t;
+    double q = fma(t2, -1.0 / 7.0 + 0.92 * 0x1p-16 / 9.0, 1.0 / 5.0);
+    q = fma(t2, q, -1.0 / 3.0);
+    const double hi = th0 + t;
+    double lo = fma(t2 * t, q, tl);
+    lo += tl0;
+    lo += t - (hi - th0);
+    return hilo{hi, lo};
+}
+
+// Quick atan for 2^-30 <= |x| <= 2^30: false where the rounding is undecided.
+SC_DDM_HD bool atan_quick(double x, double& out) {
+    const hilo v = atan_hilo(fabs(x));
+    const double r = v.hi + fma(v.hi, kAtanQuickEps, v.lo);
+    out = x < 0.0 ? -r : r;
+    return r == v.hi + fma(v.hi, -kAtanQuickEps, v.lo);
 }
 
 // Correctly rounded log and atan (the quick phase, else the full evaluation).
@@ -345,6 +331,24 @@ SC_DDM_HD double atan_dd(double x) {
     double r;
     if (a >= 9.3132257461547852e-10 && a <= 1073741824.0 && atan_quick(x, r)) return r;
     return atan_dd_full(x);
+}
+
+// The same reductions without the rounding test (the mixed form): hi + lo
+// rounded once, within 0.5001 ulp for log and atan of the arguments the
+// quick phases take (log next to 1 within an ulp).
+SC_DDM_HD double log_fast(double x) {
+    if (!(x >= 2.2250738585072014e-308 && x <= 1.7976931348623157e308)) return log(x);
+    bool exact;
+    const hilo v = log_hilo(x, exact);
+    return v.hi + v.lo;
+}
+
+SC_DDM_HD double atan_fast(double x) {
+    const double a = fabs(x);
+    if (!(a >= 9.3132257461547852e-10 && a <= 1073741824.0)) return atan(x);
+    const hilo v = atan_hilo(a);
+    const double r = v.hi + v.lo;
+    return x < 0.0 ? -r : r;
 }
 
 }  // namespace ddm

@@ -928,9 +928,9 @@ __global__ void __launch_bounds__(kThreads) k_assemble_rho(BunchConst bc, const 
 // once (sc_ddmath.cuh): correctly rounded except in rare near-tie cases, so
 // G does not carry the device library's last-bit differences into the
 // eight-corner cancellation.
-// CR: the correctly rounded double-double atan / log of the plain form;
-// otherwise CUDA's own FP64 atan / log (a few ulp), the mixed form's
-// Green's function, still FP64 throughout.
+// CR: the correctly rounded atan / log of the plain form (rounding test,
+// double-double where it cannot decide); otherwise the quick evaluations
+// rounded once (within 0.5001 ulp), the mixed form's Green's function.
 template <bool CR = true>
 __device__ __forceinline__ double igf_antiderivative(double x, double y, double z, double cellVolume) {
     double r = sqrt(x * x + y * y + z * z);
@@ -943,12 +943,12 @@ __device__ __forceinline__ double igf_antiderivative(double x, double y, double 
         tmpgrn += x * y * ddm::log_dd(z + r);
         return tmpgrn / cellVolume;
     } else {
-        double tmpgrn = -z * z * atan(x * y / (z * r)) / 2;
-        tmpgrn += -y * y * atan(x * z / (y * r)) / 2;
-        tmpgrn += -x * x * atan(y * z / (x * r)) / 2;
-        tmpgrn += y * z * log(x + r);
-        tmpgrn += x * z * log(y + r);
-        tmpgrn += x * y * log(z + r);
+        double tmpgrn = -z * z * ddm::atan_fast(x * y / (z * r)) / 2;
+        tmpgrn += -y * y * ddm::atan_fast(x * z / (y * r)) / 2;
+        tmpgrn += -x * x * ddm::atan_fast(y * z / (x * r)) / 2;
+        tmpgrn += y * z * ddm::log_fast(x + r);
+        tmpgrn += x * z * ddm::log_fast(y + r);
+        tmpgrn += x * y * ddm::log_fast(z + r);
         return tmpgrn / cellVolume;
     }
 }
