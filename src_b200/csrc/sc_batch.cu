@@ -121,7 +121,7 @@ void drop_graphs(scgpu_batch* b) {
 int variant_of(const scgpu_batch* b, int L) {
     auto it = b->fft_variant.find(L);
     if (it != b->fft_variant.end()) return it->second;
-    return (fft_register_lines() && (L == 64 || L == 128 || L == 256)) ? kFftLinesVariant : 0;
+    return (fft_register_lines() && (L == 32 || L == 64 || L == 128 || L == 256)) ? kFftLinesVariant : 0;
 }
 
 // Work tables and launch list of the current membership, uploaded to the device.
@@ -156,7 +156,13 @@ int rebuild(scgpu_batch* b) {
     };
     auto add_pass = [&](int lane, int pass) {
         std::map<int, std::vector<int>> by_len;
-        for (int i = 0; i < nm; ++i) by_len[fft_pass_length(pass, tab[i])].push_back(i);
+        for (int i = 0; i < nm; ++i) {
+            // a bunch runs either the plane kernel or the passes B, C and D
+            const bool plane = fft_pass_plane(tab[i], variant_of(b, 2 * tab[i].bc.n[0]));
+            if (pass == kPassPlane ? !plane : plane && (pass == kPassYFwd || pass == kPassXConv || pass == kPassYInv))
+                continue;
+            by_len[fft_pass_length(pass, tab[i])].push_back(i);
+        }
         for (auto& kv : by_len) {
             Launch l{lane, -1, pass, kv.first, (int)work.size(), 0, 0};
             const int v = variant_of(b, kv.first);
@@ -187,6 +193,7 @@ int rebuild(scgpu_batch* b) {
     add_pass(6, kPassYFwd);
     add_pass(3, kPassXConv);
     add_pass(3, kPassYInv);
+    add_pass(3, kPassPlane);
     add_pass(3, kPassZC2R);
     add_per_bunch(3, kBatchGrad, [&](const DevBunch& d) { return blocks_for(cells(d), 256, kCellGridCap); });
     add_per_bunch(5, kBatchGather, [](const DevBunch& d) { return d.red_blocks; });

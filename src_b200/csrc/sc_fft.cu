@@ -34,42 +34,10 @@
 #include <type_traits>
 #include <vector>
 
-#include "sc_internal.h"
+#include "sc_fft_lines.cuh"
 
 namespace sc {
 namespace {
-
-template <typename T>
-struct CT;
-template <>
-struct CT<double> {
-    using type = double2;
-};
-template <>
-struct CT<float> {
-    using type = float2;
-};
-template <typename T>
-using Cx = typename CT<T>::type;
-
-template <typename C>
-__device__ __forceinline__ C cadd(C a, C b) {
-    return {a.x + b.x, a.y + b.y};
-}
-template <typename C>
-__device__ __forceinline__ C csub(C a, C b) {
-    return {a.x - b.x, a.y - b.y};
-}
-// Complex product with its two fused multiply-adds written out.  The file is
-// compiled without FMA contraction (-fmad=false), so every kernel that shares
-// these butterflies rounds identically, whatever the surrounding code: the
-// staged, register-resident and batched transforms give the same bits.
-__device__ __forceinline__ float fmx(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fmx(double a, double b, double c) { return fma(a, b, c); }
-template <typename C>
-__device__ __forceinline__ C cmul(C a, C b) {
-    return {fmx(a.x, b.x, -(a.y * b.y)), fmx(a.x, b.y, a.y * b.x)};
-}
 
 // ---------------------------------------------------------------- cp.async
 template <int BYTES>
@@ -154,128 +122,11 @@ __host__ __device__ constexpr int threads_for(int LT) {
     return t < 32 ? 32 : t;
 }
 
-// ---------------------------------------------------------------- butterflies
-// R-point DFT in registers; forward uses exp(-2 pi i / R).
-template <typename T, int R, bool INV>
-__device__ __forceinline__ void dft(Cx<T>* v) {
-    using C = Cx<T>;
-    if constexpr (R == 2) {
-        C a = v[0], b = v[1];
-        v[0] = cadd(a, b);
-        v[1] = csub(a, b);
-    } else if constexpr (R == 4) {
-        C t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-        C t2 = cadd(v[1], v[3]), t3 = csub(v[1], v[3]);
-        v[0] = cadd(t0, t2);
-        v[2] = csub(t0, t2);
-        if constexpr (!INV) {
-            v[1] = C{t1.x + t3.y, t1.y - t3.x};
-            v[3] = C{t1.x - t3.y, t1.y + t3.x};
-        } else {
-            v[1] = C{t1.x - t3.y, t1.y + t3.x};
-            v[3] = C{t1.x + t3.y, t1.y - t3.x};
-        }
-    } else if constexpr (R == 3) {
-        const T s = INV ? (T)0.86602540378443864676 : (T)-0.86602540378443864676;
-        C t1 = cadd(v[1], v[2]);
-        C d = csub(v[1], v[2]);
-        C t2 = C{v[0].x - (T)0.5 * t1.x, v[0].y - (T)0.5 * t1.y};
-        v[0] = cadd(v[0], t1);
-        v[1] = C{t2.x - s * d.y, t2.y + s * d.x};
-        v[2] = C{t2.x + s * d.y, t2.y - s * d.x};
-    } else if constexpr (R == 8) {
-        // 2 x 4: a_k = x_k + x_{k+4}, b_k = (x_k - x_{k+4}) W8^k; X_{2m} = DFT4(a), X_{2m+1} = DFT4(b)
-        const T h = (T)0.70710678118654752440;
-        C a[4], b[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            a[k] = cadd(v[k], v[k + 4]);
-            b[k] = csub(v[k], v[k + 4]);
-        }
-        // W8^1 = (1 - i)/sqrt2 (forward), W8^2 = -i, W8^3 = -(1 + i)/sqrt2; conjugates for the inverse
-        if constexpr (!INV) {
-            b[1] = C{h * (b[1].x + b[1].y), h * (b[1].y - b[1].x)};
-            b[2] = C{b[2].y, -b[2].x};
-            b[3] = C{h * (b[3].y - b[3].x), -h * (b[3].x + b[3].y)};
-        } else {
-            b[1] = C{h * (b[1].x - b[1].y), h * (b[1].y + b[1].x)};
-            b[2] = C{-b[2].y, b[2].x};
-            b[3] = C{-h * (b[3].x + b[3].y), h * (b[3].x - b[3].y)};
-        }
-        dft<T, 4, INV>(a);
-        dft<T, 4, INV>(b);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            v[2 * m] = a[m];
-            v[2 * m + 1] = b[m];
-        }
-    } else if constexpr (R == 5) {
-        const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
-        const T s1 = INV ? (T)0.95105651629515357212 : (T)-0.95105651629515357212;
-        const T s2 = INV ? (T)0.58778525229247312917 : (T)-0.58778525229247312917;
-        C a1 = cadd(v[1], v[4]), b1 = csub(v[1], v[4]);
-        C a2 = cadd(v[2], v[3]), b2 = csub(v[2], v[3]);
-        C x0 = v[0];
-        C r1 = C{x0.x + c1 * a1.x + c2 * a2.x, x0.y + c1 * a1.y + c2 * a2.y};
-        C r2 = C{x0.x + c2 * a1.x + c1 * a2.x, x0.y + c2 * a1.y + c1 * a2.y};
-        C i1 = C{s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y};
-        C i2 = C{s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y};
-        v[0] = C{x0.x + a1.x + a2.x, x0.y + a1.y + a2.y};
-        v[1] = C{r1.x - i1.y, r1.y + i1.x};
-        v[4] = C{r1.x + i1.y, r1.y - i1.x};
-        v[2] = C{r2.x - i2.y, r2.y + i2.x};
-        v[3] = C{r2.x + i2.y, r2.y - i2.x};
-    }
-}
-
 // Shared-memory position of element i of a column: one empty slot after every
 // 8 elements.  The first Stockham stages write with strides of R elements
 // (R = 4 or 8, i.e. 64 or 128 bytes of complex double), which would put a
 // warp's stores into one or two bank groups; the skew spreads them over all.
 __host__ __device__ constexpr int sk(int i) { return i + (i >> 3); }
-
-// R-point DFT of inputs whose upper half v[R/2 .. R-1] is zero (the
-// zero-padded half of a forward transform's first stage).
-template <typename T, int R, bool INV>
-__device__ __forceinline__ void dft_half(Cx<T>* v) {
-    using C = Cx<T>;
-    if constexpr (R == 2) {
-        v[1] = v[0];
-    } else if constexpr (R == 4) {
-        const C a = v[0], b = v[1];
-        v[0] = cadd(a, b);
-        v[2] = csub(a, b);
-        if constexpr (!INV) {
-            v[1] = C{a.x + b.y, a.y - b.x};
-            v[3] = C{a.x - b.y, a.y + b.x};
-        } else {
-            v[1] = C{a.x - b.y, a.y + b.x};
-            v[3] = C{a.x + b.y, a.y - b.x};
-        }
-    } else {
-        static_assert(R == 8, "half-input DFT for radix 2, 4, 8");
-        const T h = (T)0.70710678118654752440;
-        C a[4], b[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) a[k] = b[k] = v[k];
-        if constexpr (!INV) {
-            b[1] = C{h * (b[1].x + b[1].y), h * (b[1].y - b[1].x)};
-            b[2] = C{b[2].y, -b[2].x};
-            b[3] = C{h * (b[3].y - b[3].x), -h * (b[3].x + b[3].y)};
-        } else {
-            b[1] = C{h * (b[1].x - b[1].y), h * (b[1].y + b[1].x)};
-            b[2] = C{-b[2].y, b[2].x};
-            b[3] = C{-h * (b[3].x + b[3].y), h * (b[3].x - b[3].y)};
-        }
-        dft<T, 4, INV>(a);
-        dft<T, 4, INV>(b);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            v[2 * m] = a[m];
-            v[2 * m + 1] = b[m];
-        }
-    }
-}
 
 // One Stockham autosort butterfly (radix R): butterfly j of a column reads
 // element j + r nb, r < R, applies the twiddles W^(r k step), k = j mod Ns,
@@ -579,121 +430,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_fft_x_conv(const Cx<TI>* in, 
                                                    int L1, int rows, FftPlan px, const Cx<TI>* __restrict__ twi,
                                                    const Cx<TO>* __restrict__ two) {
     fft_x_conv_body<TI, TO, LT, NC, NT, CG>(in, out, ghat, n0, n1, L1, rows, px, twi, two, blockIdx.x);
-}
-
-// ---------------------------------------------------------------- lines in registers
-// The same Stockham transform of a 64-, 128- or 256-point line (plans 8 8;
-// 4 4 8; 4 8 8: the same butterflies, twiddles and operation order as
-// block_fft, so the same bits), computed by 8 threads of one warp with the
-// data in registers: thread a holds elements a + 8m (m < L/8).  Those are
-// exactly the inputs of the first stage's butterflies a + 8q; for 128 and 256
-// points their outputs are in turn the inputs of the second stage's
-// butterflies 4a + k, which leave elements (L/8)a .. (L/8)a + L/8 - 1 in the
-// thread.  One exchange through the line's shared buffer (element p at
-// p + p/(L/8): the 8 threads' accesses fall in distinct banks) gives thread a
-// the inputs of the last stage's butterflies a + 8s, whose outputs are the
-// elements a + 8m again.  No block barrier: the 8 threads of a line are a
-// quarter of a warp.
-template <int L>
-struct LineGeo {
-    static constexpr int M = L / 8;           // elements per thread
-    static constexpr int BUF = L + 8;         // exchange buffer elements of a line
-    static constexpr int LINES = L >= 256 ? 8 : 16;  // lines per block
-    static constexpr int NT = 8 * LINES;
-};
-template <int L>
-__device__ __forceinline__ int xidx(int p) {
-    return p + p / (L / 8);
-}
-
-// BLOCK: the 8 threads of a line sit in different warps (the y passes, whose
-// lanes run along x for coalesced columns); the exchange then waits for the
-// whole block.
-template <bool BLOCK>
-__device__ __forceinline__ void line_sync() {
-    if constexpr (BLOCK)
-        __syncthreads();
-    else
-        __syncwarp();
-}
-
-template <typename T, bool INV, bool HALF_IN, int L, bool BLOCK = false>
-__device__ __forceinline__ void line_fft(Cx<T> (&v)[L / 8], int a, Cx<T>* xs, const Cx<T>* __restrict__ tw) {
-    using C = Cx<T>;
-    constexpr int M = L / 8;
-    C o[M];  // elements M a + i after the stages before the exchange
-    if constexpr (L == 64) {
-        // stage 1: radix 8, Ns = 1; butterfly a reads elements a + 8r
-        C u[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) u[r] = v[r];
-        if constexpr (HALF_IN)
-            dft_half<T, 8, INV>(u);
-        else
-            dft<T, 8, INV>(u);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) o[r] = u[r];
-    } else {
-        constexpr int R2 = L == 128 ? 4 : 8;   // second-stage radix
-        constexpr int Q = M / 4;                // first-stage butterflies per thread
-        C w[Q][4];
-        // stage 1: radix 4, Ns = 1; butterfly a + 8q reads elements a + 8q + (L/4) r
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            C u[4];
-            u[0] = v[q];
-            u[1] = v[q + Q];
-            if constexpr (HALF_IN) {
-                dft_half<T, 4, INV>(u);
-            } else {
-                u[2] = v[q + 2 * Q];
-                u[3] = v[q + 3 * Q];
-                dft<T, 4, INV>(u);
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r) w[q][r] = u[r];
-        }
-        // stage 2: radix R2, Ns = 4, step L / (4 R2) = 8; butterfly 4a + k
-        // reads the first stage's outputs 4a + k + (L/R2) r = output k of
-        // butterfly a + 8r, and writes elements M a + k + 4r
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            C u[R2];
-#pragma unroll
-            for (int r = 0; r < R2; ++r) u[r] = w[r][k];
-#pragma unroll
-            for (int r = 1; r < R2; ++r) {
-                C t = __ldg(&tw[r * k * 8]);
-                if (INV) t.y = -t.y;
-                u[r] = cmul(u[r], t);
-            }
-            dft<T, R2, INV>(u);
-#pragma unroll
-            for (int r = 0; r < R2; ++r) o[k + 4 * r] = u[r];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < M; ++i) xs[xidx<L>(M * a + i)] = o[i];
-    line_sync<BLOCK>();
-    // last stage: radix 8, Ns = M, step 1; butterfly j = a + 8s reads
-    // elements j + M r and writes them back in place
-#pragma unroll
-    for (int s2 = 0; s2 < M / 8; ++s2) {
-        const int j = a + 8 * s2;
-        C u[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L>(j + M * r)];
-#pragma unroll
-        for (int r = 1; r < 8; ++r) {
-            C t = __ldg(&tw[r * j]);
-            if (INV) t.y = -t.y;
-            u[r] = cmul(u[r], t);
-        }
-        dft<T, 8, INV>(u);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[s2 + (M / 8) * r] = u[r];  // element j + M r = a + 8 (s2 + (M/8) r)
-    }
-    line_sync<BLOCK>();  // the buffer is free again
 }
 
 // Pass C on rows of L = 2 n0 points: 8 threads per row.  The forward
@@ -1529,6 +1265,10 @@ inline bool special_length(int L) { return L == 32 || L == 64 || L == 96 || L ==
 
 bool fft_register_lines() { return register_lines(); }
 
+bool fft_pass_plane(const DevBunch& b, int variant) {
+    return variant == kFftLinesVariant && fft_plane_length(2 * b.bc.n[0], 2 * b.bc.n[1]);
+}
+
 int fft_pass_length(int pass, const DevBunch& b) {
     switch (pass) {
         case kPassZR2C:
@@ -1544,6 +1284,11 @@ int fft_pass_length(int pass, const DevBunch& b) {
 void fft_pass_grid(int pass, const DevBunch& b, int variant, int* gx, int* gy) {
     const int L = fft_pass_length(pass, b);
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
+    if (pass == kPassPlane) {  // block (rank in the cluster, plane)
+        *gx = fft_plane_cluster(L);
+        *gy = n2 + 1;
+        return;
+    }
     if (variant == kFftLinesVariant) {
         const int lines = L >= 256 ? LineGeo<256>::LINES : LineGeo<128>::LINES;
         if (line_length(L) && (pass == kPassYFwd || pass == kPassYInv)) {
@@ -1592,6 +1337,10 @@ void fft_pass_grid(int pass, const DevBunch& b, int variant, int* gx, int* gy) {
 void launch_fft_pass_batch(int pass, int L, int precision, int variant, const DevBunch* tab, const int4* work, int nitems,
                            int n, cudaStream_t s) {
     if (n <= 0 || nitems <= 0) return;
+    if (pass == kPassPlane) {
+        launch_plane_conv_batch(L, precision, tab, work, nitems, n, s);
+        return;
+    }
     if (precision == 0)
         pass_batch<double>(pass, L, variant, tab, work, nitems, n, s);
     else
@@ -1753,6 +1502,7 @@ static void convolution_t(const DevBunch& b, int mode, int parts, cudaStream_t s
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
     const int L0 = 2 * n0, L1 = 2 * n1, L2 = axis_length(b, 2);
     const int K = L2 / 2;  // half-spectrum planes 0..K along z
+    const bool plane = fft_plane_length(L0, L1);
     const FftPlan px = make_plan(L0), py = make_plan(L1), pz = make_plan(L2);
     const C* twx = reinterpret_cast<const C*>(tw_for(b, 0));
     const C* twy = reinterpret_cast<const C*>(tw_for(b, 1));
@@ -1771,11 +1521,22 @@ static void convolution_t(const DevBunch& b, int mode, int parts, cudaStream_t s
             with_length(L2, LaunchA<T, true>{(const T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s});
         else
             with_length(L2, LaunchA<T>{(const T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s});
-        with_length(L1, LaunchY<T, false>{fwd, n0, L0, n1, L1, K + 1, py, twy, s});
+        if (!plane) with_length(L1, LaunchY<T, false>{fwd, n0, L0, n1, L1, K + 1, py, twy, s});
     }
-    if ((parts & kConvRestPart) && b.periodic_z) {
-        with_length(L0, LaunchC<T, true>{fwd, inv, (const T*)b.ghat_img, n0, n1, L1, (K + 1) * L1, px, twx, twx_d, s});
+    // passes C and D, or B, C and D of a plane in one kernel
+    auto conv_cd = [&](const void* ghat, bool complex_g) {
+        if (plane) {
+            launch_plane_conv(L0, PlaneConv{fwd, inv, ghat, b.tw[0], b.tw[1], K + 1, b.precision == 0, complex_g}, s);
+            return;
+        }
+        if (complex_g)
+            with_length(L0, LaunchC<T, true>{fwd, inv, (const T*)ghat, n0, n1, L1, (K + 1) * L1, px, twx, twx_d, s});
+        else
+            with_length(L0, LaunchC<T>{fwd, inv, (const T*)ghat, n0, n1, L1, (K + 1) * L1, px, twx, twx_d, s});
         with_length(L1, LaunchY<double, true>{inv, n0, L0, L1, n1, K + 1, py, twy_d, s});
+    };
+    if ((parts & kConvRestPart) && b.periodic_z) {
+        conv_cd(b.ghat_img, true);
         if (mode == kConvSelfField)
             with_length(L2, LaunchE<true, false, true>{inv, b.phi, n0, n1, n2, L0, L1, pz, twz_d, b.st, normFact,
                                                        b.bc.coupling, s});
@@ -1785,16 +1546,14 @@ static void convolution_t(const DevBunch& b, int mode, int parts, cudaStream_t s
         return;
     }
     if (parts & kConvRestPart) {
-        with_length(L0, LaunchC<T>{fwd, inv, (const T*)b.ghat, n0, n1, L1, (n2 + 1) * L1, px, twx, twx_d, s});
-        with_length(L1, LaunchY<double, true>{inv, n0, L0, L1, n1, n2 + 1, py, twy_d, s});
+        conv_cd(b.ghat, false);
         if (mode == kConvSelfField)
             with_length(L2, LaunchE<true>{inv, b.phi, n0, n1, n2, L0, L1, pz, twz_d, b.st, normFact, b.bc.coupling, s});
         else
             with_length(L2, LaunchE<false>{inv, b.phi, n0, n1, n2, L0, L1, pz, twz_d, b.st, normFact, b.bc.coupling, s});
     }
     if (parts & kConvImagePart) {
-        with_length(L0, LaunchC<T, true>{fwd, inv, (const T*)b.ghat_img, n0, n1, L1, (n2 + 1) * L1, px, twx, twx_d, s});
-        with_length(L1, LaunchY<double, true>{inv, n0, L0, L1, n1, n2 + 1, py, twy_d, s});
+        conv_cd(b.ghat_img, true);
         if (mode == kConvSelfField)
             with_length(L2, LaunchE<true, true>{inv, b.phi, n0, n1, n2, L0, L1, pz, twz_d, b.st, normFact, b.bc.coupling, s});
         else
@@ -1822,6 +1581,7 @@ void fft_set_smem_limits() {
     sl.run<128>();
     sl.run<256>();
     sl.run<0>();
+    fft_plane_set_limits();
 }
 
 }  // namespace sc

@@ -199,6 +199,7 @@ enum : int {
     kPassYFwd,       // B
     kPassXConv,      // C
     kPassYInv,       // D
+    kPassPlane,      // B, C and D in one kernel (sc_fft_plane.cu)
     kPassZC2R,       // E (self-field scaling)
     kPassDctZ,
     kPassDctY,
@@ -212,6 +213,8 @@ bool fft_register_lines();           // line transforms enabled (SCGPU_FFT_LINES
 void fft_pass_grid(int pass, const DevBunch& b, int variant, int* gx, int* gy);
 // Transform length of a pass's axis for a bunch.
 int fft_pass_length(int pass, const DevBunch& b);
+// whether the bunch's passes B, C, D run as the plane kernel with this tile-shape variant
+bool fft_pass_plane(const DevBunch& b, int variant);
 void launch_fft_pass_batch(int pass, int L, int precision, int variant, const DevBunch* tab, const int4* items,
                            int nitems, int nblocks, cudaStream_t s);
 
@@ -219,6 +222,25 @@ void launch_fft_pass_batch(int pass, int L, int precision, int variant, const De
 long long scan_scratch_ints(long long n);
 void exclusive_scan(const int* in, int* out, long long n, int* blocks, cudaStream_t s);
 void launch_sort(const DevBunch& b, cudaStream_t s);
+
+// Plane kernels (sc_fft_plane.cu): passes B, C and D of a kz plane in one
+// kernel on a cluster of blocks, for n0 == n1 with a line length that fits
+// (32, 64, 128 points; off with SCGPU_FFT_LINES=0).
+struct PlaneConv {
+    const void* in;    // pass A's half spectrum (complex T)
+    double2* out;      // after the inverse y transform; may be `in` (plain form)
+    const void* ghat;  // spectrum of G: real T, or complex T with complex_g
+    const void* tw0;   // twiddle tables of x and y: doubles, then floats
+    const void* tw1;
+    int planes;        // kz planes
+    bool f64, complex_g;
+};
+bool fft_plane_length(int L0, int L1);
+int fft_plane_cluster(int L);  // blocks per plane
+void launch_plane_conv(int L, const PlaneConv& c, cudaStream_t s);
+void launch_plane_conv_batch(int L, int precision, const DevBunch* tab, const int4* items, int nitems, int nblocks,
+                             cudaStream_t s);
+void fft_plane_set_limits();
 
 // FFT TU (sc_fft.cu)
 void launch_green_transform(const DevBunch& b, cudaStream_t s);
