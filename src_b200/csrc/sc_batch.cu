@@ -157,10 +157,12 @@ int rebuild(scgpu_batch* b) {
     auto add_pass = [&](int lane, int pass) {
         std::map<int, std::vector<int>> by_len;
         for (int i = 0; i < nm; ++i) {
-            // a bunch runs either the plane kernel or the passes B, C and D
+            // a bunch runs either the plane kernels or the passes B, C, D and the y and x cosine transforms
             const bool plane = fft_pass_plane(tab[i], variant_of(b, 2 * tab[i].bc.n[0]));
-            if (pass == kPassPlane ? !plane : plane && (pass == kPassYFwd || pass == kPassXConv || pass == kPassYInv))
-                continue;
+            const bool on_planes = pass == kPassPlane || pass == kPassDctPlane;
+            const bool replaced = pass == kPassYFwd || pass == kPassXConv || pass == kPassYInv || pass == kPassDctY ||
+                                  pass == kPassDctX;
+            if (plane ? replaced : on_planes) continue;
             by_len[fft_pass_length(pass, tab[i])].push_back(i);
         }
         for (auto& kv : by_len) {
@@ -186,6 +188,7 @@ int rebuild(scgpu_batch* b) {
     add_pass(1, kPassDctZ);
     add_pass(1, kPassDctY);
     add_pass(1, kPassDctX);
+    add_pass(1, kPassDctPlane);
     add_per_bunch(2, kBatchDeposit, [dep](const DevBunch& d) { return blocks_for(d.bc.N, dep, 148 * 8 * 256 / dep); });
     add_per_bunch(2, kBatchAssemble, [&](const DevBunch& d) { return blocks_for(cells(d), 256, kCellGridCap); });
     add_per_bunch(4, kBatchAdvance, [](const DevBunch&) { return 1; });

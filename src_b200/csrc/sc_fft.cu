@@ -1046,7 +1046,9 @@ struct LaunchDct {
     }
     template <int LT, int V>
     void go() {
-        constexpr int NC = Geo<LT, V>::NC, NT = Geo<LT, V>::NT;
+        // forming G reads eight values per element, so the z pass takes 256
+        // threads to stage its tile, however few its butterflies need
+        constexpr int NC = Geo<LT, V>::NC, NT = FROM_TMP ? 256 : Geo<LT, V>::NT;
         dim3 g((unsigned)((nb + 2 * NC - 1) / (2 * NC)), (unsigned)outer);
         k_dct_lines<TO, LT, NC, NT, FROM_TMP><<<g, NT, smem_of<double2>(pl.L, NC), s>>>(in, out, len, nb, sb, so, se, pl,
                                                                                      tw, t0, t1);
@@ -1082,7 +1084,7 @@ struct SetLimits {
         allow(k_fft_z_c2r<double, false, LT, NC, NT>);
         allow(k_dct_lines<double, LT, NC, NT>);
         allow(k_dct_lines<float, LT, NC, NT>);
-        allow(k_dct_lines<double, LT, NC, NT, true>);
+        allow(k_dct_lines<double, LT, NC, 256, true>);
         allow(k_fft_x_conv<double, double, LT, NC, NT, true>);
         allow(k_fft_x_conv<float, double, LT, NC, NT, true>);
         allow(k_fft_z_c2r<double, true, LT, NC, NT, true>);
@@ -1289,6 +1291,11 @@ void fft_pass_grid(int pass, const DevBunch& b, int variant, int* gx, int* gy) {
         *gy = n2 + 1;
         return;
     }
+    if (pass == kPassDctPlane) {
+        *gx = n2 + 1;
+        *gy = 1;
+        return;
+    }
     if (variant == kFftLinesVariant) {
         const int lines = L >= 256 ? LineGeo<256>::LINES : LineGeo<128>::LINES;
         if (line_length(L) && (pass == kPassYFwd || pass == kPassYInv)) {
@@ -1339,6 +1346,10 @@ void launch_fft_pass_batch(int pass, int L, int precision, int variant, const De
     if (n <= 0 || nitems <= 0) return;
     if (pass == kPassPlane) {
         launch_plane_conv_batch(L, precision, tab, work, nitems, n, s);
+        return;
+    }
+    if (pass == kPassDctPlane) {
+        launch_dct_plane_batch(L, precision, tab, work, nitems, n, s);
         return;
     }
     if (precision == 0)
@@ -1404,46 +1415,56 @@ static inline const void* tw_for(const DevBunch& b, int d) {
     return b.precision == 0 ? (const void*)dptr : (const void*)(dptr + L);
 }
 
-// Spectrum of the mirrored G from b.gline ((n0+1)(n1+1)(n2+1), FP64), into b.ghat.
-void launch_green_transform(const DevBunch& b, cudaStream_t s) {
-    const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
-    const long long g0 = n0 + 1, g1 = n1 + 1, g2 = n2 + 1;
-    const FftPlan p0 = make_plan(2 * n0), p1 = make_plan(2 * n1), p2 = make_plan(2 * n2);
+// Cosine transforms of `planes` planes of (n0+1)(n1+1) reals along y (in to
+// tmp) and x (tmp to out), or both in one kernel per plane (in to out).
+template <typename TO>
+static void dct_yx(const DevBunch& b, const double* in, double* tmp, TO* out, int planes, cudaStream_t s) {
+    const int n0 = b.bc.n[0], n1 = b.bc.n[1];
+    const long long g0 = n0 + 1, g1 = n1 + 1;
+    if (fft_plane_length(2 * n0, 2 * n1)) {
+        launch_dct_plane(2 * n0, in, out, sizeof(TO) == sizeof(double), planes, b.tw[1], b.tw[0], s);
+        return;
+    }
+    const FftPlan p0 = make_plan(2 * n0), p1 = make_plan(2 * n1);
     const double2* tw0 = reinterpret_cast<const double2*>(b.tw[0]);
     const double2* tw1 = reinterpret_cast<const double2*>(b.tw[1]);
+    // y lines: batch x, outer z
+    with_length(2 * n1, LaunchDct<double>{in, tmp, (int)g1, (int)g0, planes, 1, g0 * g1, g0, p1, tw1, s});
+    // x lines: batch y (stride g0), outer z
+    with_length(2 * n0, LaunchDct<TO>{tmp, out, (int)g0, (int)g1, planes, g0, g0 * g1, 1, p0, tw0, s});
+}
+
+// Spectrum of the mirrored G from b.gline ((n0+1)(n1+1)(n2+1), FP64), into b.ghat.
+void launch_green_transform(const DevBunch& b, cudaStream_t s) {
+    const long long g0 = b.bc.n[0] + 1, g1 = b.bc.n[1] + 1, g2 = b.bc.n[2] + 1;
+    const FftPlan p2 = make_plan(2 * b.bc.n[2]);
     const double2* tw2 = reinterpret_cast<const double2*>(b.tw[2]);
     // z lines: batch x (stride 1), outer y
-    with_length(2 * n2, LaunchDct<double>{b.gline, b.gtmp, (int)g2, (int)g0, (int)g1, 1, g0, g0 * g1, p2, tw2, s});
-    // y lines: batch x, outer z
-    with_length(2 * n1, LaunchDct<double>{b.gtmp, b.gline, (int)g1, (int)g0, (int)g2, 1, g0 * g1, g0, p1, tw1, s});
-    // x lines: batch y (stride g0), outer z
+    with_length(p2.L, LaunchDct<double>{b.gline, b.gtmp, (int)g2, (int)g0, (int)g1, 1, g0, g0 * g1, p2, tw2, s});
     if (b.precision == 0)
-        with_length(2 * n0, LaunchDct<double>{b.gline, (double*)b.ghat, (int)g0, (int)g1, (int)g2, g0, g0 * g1, 1, p0, tw0, s});
+        dct_yx(b, b.gtmp, b.gline, (double*)b.ghat, (int)g2, s);
     else
-        with_length(2 * n0, LaunchDct<float>{b.gline, (float*)b.ghat, (int)g0, (int)g1, (int)g2, g0, g0 * g1, 1, p0, tw0, s});
+        dct_yx(b, b.gtmp, b.gline, (float*)b.ghat, (int)g2, s);
 }
 
 // The same spectrum from the antiderivative (b.gtmp, launch_igf_tmp): the
 // z transforms form G as they stage it and write gline, the y transforms
-// gline -> gtmp, the x transforms gtmp -> ghat.  G's values and every
-// transform are those of launch_igf + launch_green_transform, so Ĝ has the
-// same bits; G is never stored.
+// gline -> gtmp, the x transforms gtmp -> ghat (or both gline -> ghat).  G's
+// values and every transform are those of launch_igf +
+// launch_green_transform, so Ĝ has the same bits; G is never stored.
 void launch_green_transform_from_tmp(const DevBunch& b, cudaStream_t s) {
-    const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
-    const long long g0 = n0 + 1, g1 = n1 + 1, g2 = n2 + 1;
-    const FftPlan p0 = make_plan(2 * n0), p1 = make_plan(2 * n1), p2 = make_plan(2 * n2);
-    const double2* tw0 = reinterpret_cast<const double2*>(b.tw[0]);
-    const double2* tw1 = reinterpret_cast<const double2*>(b.tw[1]);
+    const int n0 = b.bc.n[0], n1 = b.bc.n[1];
+    const long long g0 = n0 + 1, g1 = n1 + 1, g2 = b.bc.n[2] + 1;
+    const FftPlan p2 = make_plan(2 * b.bc.n[2]);
     const double2* tw2 = reinterpret_cast<const double2*>(b.tw[2]);
     LaunchDct<double, true> z{b.gtmp, b.gline, (int)g2, (int)g0, (int)g1, 1, g0, g0 * g1, p2, tw2, s};
     z.t0 = n0 + 2;
     z.t1 = n1 + 2;
-    with_length(2 * n2, z);
-    with_length(2 * n1, LaunchDct<double>{b.gline, b.gtmp, (int)g1, (int)g0, (int)g2, 1, g0 * g1, g0, p1, tw1, s});
+    with_length(p2.L, z);
     if (b.precision == 0)
-        with_length(2 * n0, LaunchDct<double>{b.gtmp, (double*)b.ghat, (int)g0, (int)g1, (int)g2, g0, g0 * g1, 1, p0, tw0, s});
+        dct_yx(b, b.gline, b.gtmp, (double*)b.ghat, (int)g2, s);
     else
-        with_length(2 * n0, LaunchDct<float>{b.gtmp, (float*)b.ghat, (int)g0, (int)g1, (int)g2, g0, g0 * g1, 1, p0, tw0, s});
+        dct_yx(b, b.gline, b.gtmp, (float*)b.ghat, (int)g2, s);
 }
 
 // Spectrum of the image's shifted G (b.gimg, (n0+1)(n1+1)(2 n2), FP64):
@@ -1454,21 +1475,18 @@ void launch_green_transform_image(const DevBunch& b, cudaStream_t s) {
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
     const long long g0 = n0 + 1, g1 = n1 + 1, L2 = 2 * n2;
     const long long GI = g0 * g1 * L2;
-    const FftPlan p0 = make_plan(2 * n0), p1 = make_plan(2 * n1), p2 = make_plan(2 * n2);
-    const double2* tw0 = reinterpret_cast<const double2*>(b.tw[0]);
-    const double2* tw1 = reinterpret_cast<const double2*>(b.tw[1]);
+    const FftPlan p2 = make_plan(2 * n2);
     const double2* tw2 = reinterpret_cast<const double2*>(b.tw[2]);
     double* ga = b.gimg;
     double* gb = b.gimg + GI;
-    // y lines: batch x, outer z (2 n2 planes)
-    with_length(2 * n1, LaunchDct<double>{ga, gb, (int)g1, (int)g0, (int)L2, 1, g0 * g1, g0, p1, tw1, s});
-    // x lines: batch y (stride g0), outer z
-    with_length(2 * n0, LaunchDct<double>{gb, ga, (int)g0, (int)g1, (int)L2, g0, g0 * g1, 1, p0, tw0, s});
+    const bool plane = fft_plane_length(2 * n0, 2 * n1);
+    double* go = plane ? gb : ga;  // the plane kernel does not work in place
+    dct_yx(b, ga, gb, go, (int)L2, s);
     // z lines of length 2 n2: batch (x, y), element stride g0 g1
     if (b.precision == 0)
-        with_length(2 * n2, LaunchRfftNeg<double>{ga, (double2*)b.ghat_img, (int)(g0 * g1), g0 * g1, p2, tw2, s});
+        with_length(2 * n2, LaunchRfftNeg<double>{go, (double2*)b.ghat_img, (int)(g0 * g1), g0 * g1, p2, tw2, s});
     else
-        with_length(2 * n2, LaunchRfftNeg<float>{ga, (float2*)b.ghat_img, (int)(g0 * g1), g0 * g1, p2, tw2, s});
+        with_length(2 * n2, LaunchRfftNeg<float>{go, (float2*)b.ghat_img, (int)(g0 * g1), g0 * g1, p2, tw2, s});
 }
 
 // Periodic z (FFTPoissonSolver with bcz, :130-155, :661-662): G on its first
@@ -1478,16 +1496,15 @@ void launch_green_transform_image(const DevBunch& b, cudaStream_t s) {
 void launch_green_transform_periodic(const DevBunch& b, cudaStream_t s) {
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
     const long long g0 = n0 + 1, g1 = n1 + 1;
-    const FftPlan p0 = make_plan(2 * n0), p1 = make_plan(2 * n1), pz = make_plan(n2);
-    const double2* tw0 = reinterpret_cast<const double2*>(b.tw[0]);
-    const double2* tw1 = reinterpret_cast<const double2*>(b.tw[1]);
+    const FftPlan pz = make_plan(n2);
     const double2* tw2 = reinterpret_cast<const double2*>(b.tw[2]);
-    with_length(2 * n1, LaunchDct<double>{b.gline, b.gtmp, (int)g1, (int)g0, n2, 1, g0 * g1, g0, p1, tw1, s});
-    with_length(2 * n0, LaunchDct<double>{b.gtmp, b.gline, (int)g0, (int)g1, n2, g0, g0 * g1, 1, p0, tw0, s});
+    const bool plane = fft_plane_length(2 * n0, 2 * n1);
+    double* go = plane ? b.gtmp : b.gline;
+    dct_yx(b, b.gline, b.gtmp, go, n2, s);
     if (b.precision == 0)
-        with_length(n2, LaunchRfftNeg<double, false>{b.gline, (double2*)b.ghat_img, (int)(g0 * g1), g0 * g1, pz, tw2, s});
+        with_length(n2, LaunchRfftNeg<double, false>{go, (double2*)b.ghat_img, (int)(g0 * g1), g0 * g1, pz, tw2, s});
     else
-        with_length(n2, LaunchRfftNeg<float, false>{b.gline, (float2*)b.ghat_img, (int)(g0 * g1), g0 * g1, pz, tw2, s});
+        with_length(n2, LaunchRfftNeg<float, false>{go, (float2*)b.ghat_img, (int)(g0 * g1), g0 * g1, pz, tw2, s});
 }
 
 // T is the type of the forward half (A, B and the forward x transform of C);

@@ -204,6 +204,7 @@ enum : int {
     kPassDctZ,
     kPassDctY,
     kPassDctX,
+    kPassDctPlane,   // the y and x cosine transforms in one kernel
     kNumPasses
 };
 constexpr int kFftVariants = 5;
@@ -240,6 +241,12 @@ int fft_plane_cluster(int L);  // blocks per plane
 void launch_plane_conv(int L, const PlaneConv& c, cudaStream_t s);
 void launch_plane_conv_batch(int L, int precision, const DevBunch* tab, const int4* items, int nitems, int nblocks,
                              cudaStream_t s);
+// the cosine transforms of `planes` planes of (n0+1)(n1+1) reals along y and
+// x, `in` to `out` (double, or float with out_f64 false); tw1, tw0: the y and x tables
+void launch_dct_plane(int L, const double* in, void* out, bool out_f64, int planes, const void* tw1, const void* tw0,
+                      cudaStream_t s);
+void launch_dct_plane_batch(int L, int precision, const DevBunch* tab, const int4* items, int nitems, int nblocks,
+                            cudaStream_t s);
 void fft_plane_set_limits();
 
 // FFT TU (sc_fft.cu)
