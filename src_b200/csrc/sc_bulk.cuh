@@ -58,22 +58,4 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
     return false;
 }
 
-// Stages element range [first, first + count) of up to three double arrays
-// into shared memory: thread 0 issues the copies of the 16-byte aligned body
-// (an even number of elements when `first` is even) and arms the barrier;
-// the last element of an odd count is not copied (callers load it from
-// global memory).  Returns the number of elements staged.
-template <int NA>
-__device__ __forceinline__ long long stage_doubles(double* const (&dst)[NA], const double* const (&src)[NA],
-                                                   long long first, long long count, uint64_t* bar) {
-    const long long body = count & ~1ll;
-    if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(bar, (unsigned)(NA * body * sizeof(double)));
-        if (body > 0)
-#pragma unroll
-            for (int a = 0; a < NA; ++a) bulk_g2s(dst[a], src[a] + first, (unsigned)(body * sizeof(double)), bar);
-    }
-    return body;
-}
-
 }  // namespace sc

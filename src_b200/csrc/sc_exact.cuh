@@ -32,6 +32,50 @@ __device__ __forceinline__ i128 ex_from(double v) {
     return (bits >> 63) ? -(i128)mag : (i128)mag;
 }
 
+// The same fixed point accumulated per thread in two 64-bit words, value
+// hi 2^36 + lo in units of 2^-72, for |v| < 2^10: hi gains floor(|v| 2^36)
+// and lo the next 36 bits, each with v's sign.  Adding 2^16 (2^-20) with
+// rounding towards zero leaves the bits above 2^-36 (2^-72) in the
+// mantissa field, so two additions and two subtractions replace the 128-bit
+// shift and addition of ex_from (about 18 operations per value against 35).
+// hi grows by less than 2^46 per value, lo by less than 2^36: 2^16 values per
+// thread fit.  Larger values (and NaN) go to `big`, four 64-bit counters per value in
+// shared memory that take the 32-bit chunks of ex_from's integer.
+struct ExAcc {
+    long long hi, lo;
+};
+
+// All NV values at once: the rare path appears once in the caller's code.
+template <int NV>
+__device__ __forceinline__ void ex_add(ExAcc (&acc)[NV], const double (&v)[NV], unsigned long long* big) {
+    bool fits = true;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) fits = fits && fabs(v[k]) < 1024.0;
+    if (fits) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const double a = fabs(v[k]);
+            const double m = __dadd_rz(a, 0x1p16);
+            const double q = __dadd_rz(a - (m - 0x1p16), 0x1p-20);
+            const long long sign = __double_as_longlong(v[k]) >> 63;
+            acc[k].hi += ((__double_as_longlong(m) & 0xfffffffffffffll) ^ sign) - sign;
+            acc[k].lo += ((__double_as_longlong(q) & 0xfffffffffffffll) ^ sign) - sign;
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < NV; ++k) {
+            double x = v[0];
+#pragma unroll
+            for (int j = 1; j < NV; ++j) x = k == j ? v[j] : x;
+            const u128 t = (u128)ex_from(x);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) atomicAdd(big + 4 * k + j, (unsigned long long)(unsigned)(t >> (32 * j)));
+        }
+    }
+}
+
+__device__ __forceinline__ i128 ex_value(const ExAcc& acc) { return ((i128)acc.hi << 36) + (i128)acc.lo; }
+
 // correctly rounded double of x * 2^-kExFrac
 __device__ __forceinline__ double ex_to_double(i128 x) {
     const bool neg = x < 0;
