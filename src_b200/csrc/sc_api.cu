@@ -1371,6 +1371,10 @@ int scgpu_track(scgpu_ctx* c, int nsteps, double* stats) {
     const bool want = stats != nullptr;
     cudaStream_t s = c->stream;
     CK(cudaEventRecord(c->ev_t0, s));
+    // the steps of this call hand each other pushed positions; a statistics
+    // record needs them unpushed at the end of every step
+    if (nsteps > 1 && !want)
+        CK(cudaMemcpyAsync(&c->b.st->left, &nsteps, sizeof(int), cudaMemcpyHostToDevice, s));
     for (int k = 0; k < nsteps; ++k) {
         const bool reorder = c->reorder_every > 0 && (c->steps_done % c->reorder_every) == 0;
         if (c->use_graphs && (!c->xfn || c->xcapturable)) {

@@ -37,6 +37,11 @@ __global__ void k_collect_flags(const DevBunch* __restrict__ tab, int n, int* __
     }
 }
 
+__global__ void k_set_left(const DevBunch* __restrict__ tab, int n, int steps) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) tab[i].st->left = steps;
+}
+
 int blocks_for(long long work, int threads, int cap) {
     long long g = (work + threads - 1) / threads;
     if (g < 1) g = 1;
@@ -282,6 +287,8 @@ int launch(scgpu_batch* b, int nsteps) {
     b->in_flight = nsteps;
     if (b->members.empty()) return SCGPU_OK;
     BCK(cudaEventRecord(b->ev_t0, b->stream));
+    const int nm = (int)b->members.size();
+    if (nsteps > 1) k_set_left<<<(nm + 127) / 128, 128, 0, b->stream>>>(b->d_tab, nm, nsteps);
     for (int k = 0; k < nsteps; ++k) {
         const bool reorder = b->reorder_every > 0 && (b->steps % b->reorder_every) == 0;
         cudaGraphExec_t& gx = b->graphs[reorder ? 1 : 0];

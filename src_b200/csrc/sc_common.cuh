@@ -90,6 +90,11 @@ struct StepState {
     double zshift;      // z shift of the image's Green's function (PartBunch.cpp:249)
     long long bin_count;  // particles in the bin (per-bin copies)
     int binned;         // the energy-bin loop is on: Q is restored after the scatter (ParallelTTracker.cpp:576)
+    // the first half drift of a step runs at the end of the gather of the
+    // step before when both belong to one call: steps left in the call (this
+    // one included), and whether the positions have had their first half drift
+    int left;
+    int pushed;
     int pad_;
     // sharded bunch: this rank's partial results, combined over the ranks
     // between kernels (bounds by min; exact sums as 32-bit chunks of the
@@ -826,23 +831,25 @@ SC_HD double wrap_z(double t, double lo, double hi) {
     return t;
 }
 
-// push_one with s = c dt and rs = RN(1/s) precomputed: same results.
-SC_HD void push_r(double* R, const double* P, double s, double rs) {
+// push_one in two parts: the unitless step 0.5 P / gamma, and R moved by it
+// (s = c dt, rs = RN(1/s) precomputed); together the same results.
+SC_HD void push_step(const double* P, double* step) {
     bool fast = true;
-    double r0 = div_rcp_nc(R[0], s, rs, fast), r1 = div_rcp_nc(R[1], s, rs, fast), r2 = div_rcp_nc(R[2], s, rs, fast);
     const double g = sqrt(1.0 + dot3(P, P));
     const double rg = 1.0 / g;
-    r0 += div_rcp_nc(0.5 * P[0], g, rg, fast);
-    r1 += div_rcp_nc(0.5 * P[1], g, rg, fast);
-    r2 += div_rcp_nc(0.5 * P[2], g, rg, fast);
-    if (!fast) {
-        r0 = R[0] / s + 0.5 * P[0] / g;
-        r1 = R[1] / s + 0.5 * P[1] / g;
-        r2 = R[2] / s + 0.5 * P[2] / g;
-    }
-    R[0] = r0 * s;
-    R[1] = r1 * s;
-    R[2] = r2 * s;
+    double q[3];
+    for (int d = 0; d < 3; ++d) q[d] = div_rcp_nc(0.5 * P[d], g, rg, fast);
+    if (!fast)
+        for (int d = 0; d < 3; ++d) q[d] = 0.5 * P[d] / g;
+    for (int d = 0; d < 3; ++d) step[d] = q[d];
+}
+SC_HD void push_move(double* R, const double* step, double s, double rs) {
+    bool fast = true;
+    double q[3];
+    for (int d = 0; d < 3; ++d) q[d] = div_rcp_nc(R[d], s, rs, fast);
+    if (!fast)
+        for (int d = 0; d < 3; ++d) q[d] = R[d] / s;
+    for (int d = 0; d < 3; ++d) R[d] = (q[d] + step[d]) * s;
 }
 
 // kick_one with ke = 0.5 dt q c / m and ktn = 0.5 dt q c c precomputed.

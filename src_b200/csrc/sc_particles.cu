@@ -8,7 +8,7 @@
 // its fused multiply-adds explicitly.
 //
 //   k_reduce_state       momentum sums (+ beam statistics) and the beam frame
-//   k_drift_to_beam      half drift, reference -> beam frame, bounds, mesh
+//   k_drift_to_beam      half drift (a call's first step), reference -> beam frame, bounds, mesh
 //   k_advance_reference  reference particle and frame update (one thread)
 //   k_cell_keys          CIC cell key and rank in its cell (counting sort for the reorder)
 //   k_deposit            warp groups by cell, exact group sums, exact integer node sums
@@ -16,7 +16,8 @@
 //   k_igf_tmp, k_igf_G   integrated Green's function (FFTPoissonSolver.cpp:459-522)
 //   k_grad               -Grad phi (UniformCartesian.hpp:2129-2203), boost scaling
 //   k_gather_kick_push   CIC gather, B from E, back to the reference frame, Boris
-//                        kick, half drift, reference-frame update, momentum sums
+//                        kick, half drift, reference-frame update, momentum sums, the
+//                        next step's first half drift
 //   k_gather_staged      the same with the particle state streamed through shared
 //                        memory by bulk copies (cp.async.bulk, mbarrier), the default
 #include <cstdio>
@@ -299,17 +300,32 @@ __device__ __forceinline__ void cross_fma(const double* a, const double* b, doub
     r[2] = r2;
 }
 
-// MIXED: the mixed form's half drift R += (c dt / 2) P / gamma and beam-frame
-// translation and rotation in fused multiply-adds (the half drift of its
-// gather), in place of the reference's unitless round trip.
+// The mixed form's half drift R += (c dt / 2) P / gamma in fused
+// multiply-adds, in place of the reference's unitless round trip.
+__device__ __forceinline__ double mixed_push_factor(const double* P, double s_cdt) {
+    return (0.5 * s_cdt) / sqrt(fma(P[0], P[0], fma(P[1], P[1], fma(P[2], P[2], 1.0))));
+}
+__device__ __forceinline__ void mixed_push(double* R, double f, const double* P) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) R[a] = fma(f, P[a], R[a]);
+}
+
+// Half drift (unless the gather of the step before has done it: then P is not
+// read, 48 instead of 72 bytes per particle), reference -> beam frame, bounds,
+// mesh.  MIXED: mixed_push and the frame change in fused multiply-adds.
 template <bool DRIFT, bool MIXED = false>
 __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restrict__ x, double* __restrict__ y,
                                            double* __restrict__ z, const double* __restrict__ px,
                                            const double* __restrict__ py, const double* __restrict__ pz, StepState* st,
                                            double* partials, unsigned* ticket, VB g) {
     __shared__ Trafo r2b_s;
-    if (threadIdx.x == 0) r2b_s = st->r2b;
+    __shared__ int pushed_s;
+    if (threadIdx.x == 0) {
+        r2b_s = st->r2b;
+        pushed_s = st->pushed;
+    }
     __syncthreads();
+    const bool push = DRIFT && pushed_s == 0;  // else the gather of the step before has pushed R
     double v[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};  // min x,y,z, -max x,y,z
     // The next particle's loads are issued before the current one is
     // computed, so each thread keeps two particles' reads in flight.
@@ -318,7 +334,7 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
     double Rn[3] = {0.0, 0.0, 0.0}, Pn[3] = {0.0, 0.0, 0.0};
     if (i < bc.N) {
         Rn[0] = x[i], Rn[1] = y[i], Rn[2] = z[i];
-        if constexpr (DRIFT) Pn[0] = px[i], Pn[1] = py[i], Pn[2] = pz[i];
+        if (push) Pn[0] = px[i], Pn[1] = py[i], Pn[2] = pz[i];
     }
     for (; i < bc.N; i += stride) {
         double R[3] = {Rn[0], Rn[1], Rn[2]};
@@ -326,19 +342,21 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
         const long long j = i + stride;
         if (j < bc.N) {
             Rn[0] = x[j], Rn[1] = y[j], Rn[2] = z[j];
-            if constexpr (DRIFT) Pn[0] = px[j], Pn[1] = py[j], Pn[2] = pz[j];
+            if (push) Pn[0] = px[j], Pn[1] = py[j], Pn[2] = pz[j];
         }
         if constexpr (DRIFT) {
             double b[3];
             if constexpr (MIXED) {
-                const double gm = sqrt(fma(P[0], P[0], fma(P[1], P[1], fma(P[2], P[2], 1.0))));
-                const double hv = (0.5 * bc.s_cdt) / gm;
+                if (push) mixed_push(R, mixed_push_factor(P, bc.s_cdt), P);
                 const Trafo* t = fresh(&r2b_s);
-                const double X[3] = {fma(hv, P[0], R[0]) - t->origin[0], fma(hv, P[1], R[1]) - t->origin[1],
-                                     fma(hv, P[2], R[2]) - t->origin[2]};
+                const double X[3] = {R[0] - t->origin[0], R[1] - t->origin[1], R[2] - t->origin[2]};
                 matvec_fma(t->M, X, b);
             } else {
-                push_r(R, P, bc.s_cdt, bc.rs_cdt);
+                if (push) {
+                    double step[3];
+                    push_step(P, step);
+                    push_move(R, step, bc.s_cdt, bc.rs_cdt);
+                }
                 trafo_transform_to(*fresh(&r2b_s), R, b);
             }
             R[0] = b[0];
@@ -1461,8 +1479,8 @@ __device__ __forceinline__ void cic_gather_f32(const float* __restrict__ E4, con
 // returns false when the CIC stencil left the mesh
 template <bool EXT>
 __device__ __forceinline__ bool mixed_particle(const BunchConst& bc, const MeshConsts& m, const float* __restrict__ E4,
-                                               const Trafo& b2r, const Trafo& upd, bool upd_shift, double betaC,
-                                               const StepState* st, double* R, double* P) {
+                                               const Trafo& b2r, const Trafo& upd, bool upd_shift, bool push_next,
+                                               double betaC, const StepState* st, double* R, double* P) {
     int l[3];
     float d[3], e[3];
     const bool ok = cic_locate_fast(m.rhr, m.org, bc.n, R, l, d, bc.pz);
@@ -1496,16 +1514,15 @@ __device__ __forceinline__ bool mixed_particle(const BunchConst& bc, const MeshC
 #pragma unroll
     for (int a = 0; a < 3; ++a) P[a] = fma(ke, Ef[a], P[a] + c[a]);
     // half drift
-    const double g = sqrt(fma(P[0], P[0], fma(P[1], P[1], fma(P[2], P[2], 1.0))));
-    const double hv = (0.5 * bc.s_cdt) / g;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) Rr[a] = fma(hv, P[a], Rr[a]);
+    const double hv = mixed_push_factor(P, bc.s_cdt);
+    mixed_push(Rr, hv, P);
     // reference-frame update
     double Y[3] = {Rr[0] - upd.origin[0], Rr[1] - upd.origin[1], Rr[2] - upd.origin[2]};
     if (upd_shift) {
         R[0] = Y[0];
         R[1] = Y[1];
         R[2] = Y[2];
+        if (push_next) mixed_push(R, hv, P);  // P is unchanged: the factor too
         return ok;
     }
     matvec_fma(upd.M, Y, R);
@@ -1514,6 +1531,7 @@ __device__ __forceinline__ bool mixed_particle(const BunchConst& bc, const MeshC
     P[0] = Pu[0];
     P[1] = Pu[1];
     P[2] = Pu[2];
+    if (push_next) mixed_push(R, mixed_push_factor(P, bc.s_cdt), P);
     return ok;
 }
 
@@ -1540,6 +1558,7 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
     __shared__ Trafo b2r_s, upd_s;
     __shared__ MeshConsts ms;
     __shared__ double betaC_s;
+    __shared__ int left_s;
     __shared__ unsigned long long big[3 * 4];
     __shared__ __align__(8) uint64_t bar[STAGED ? 2 * kWarps : 1];
     load_mesh_consts(ms, st);
@@ -1548,6 +1567,7 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
         b2r_s = st->b2r;
         upd_s = st->upd;
         betaC_s = st->betaC;
+        left_s = st->left;
         if constexpr (STAGED) {
             for (int k = 0; k < 2 * kWarps; ++k) mbar_init(&bar[k], 1);
             mbar_fence_init();
@@ -1557,6 +1577,7 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
     // on a straight beamline the reference particle stays on the z axis and
     // its frame update only translates: M is exactly the identity
     const bool upd_shift = is_identity(upd_s.M);
+    const bool push_next = left_s > 1;  // the next step of this call: its first half drift here
     ExAcc acc[3] = {{0, 0}, {0, 0}, {0, 0}};
     bool bad = false;
     // one particle: state X, P in, new state out to slot i
@@ -1566,7 +1587,7 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
         if constexpr (sizeof(T) == sizeof(float) && !BINNED) {
             double R[3] = {X[0], X[1], X[2]};
             if (!mixed_particle<EXT>(bc, *fresh(&ms), reinterpret_cast<const float*>(E4), *fresh(&b2r_s),
-                                     *fresh(&upd_s), upd_shift, *fresh(&betaC_s), st, R, P))
+                                     *fresh(&upd_s), upd_shift, push_next, *fresh(&betaC_s), st, R, P))
                 bad = true;
             Ru[0] = R[0], Ru[1] = R[1], Ru[2] = R[2];
             Pu[0] = P[0], Pu[1] = P[1], Pu[2] = P[2];
@@ -1594,7 +1615,9 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
             if constexpr (EXT)
                 add_external_fields(bc.sol, bc.nsol, st->ref_to_lab_step, R, st->t_step + 0.5 * bc.dT, Ef, Bf);
             kick_r(P, Ef, Bf, bc.ke, bc.ktn, bc.mass);
-            push_r(R, P, bc.s_cdt, bc.rs_cdt);
+            double step[3];
+            push_step(P, step);
+            push_move(R, step, bc.s_cdt, bc.rs_cdt);
             const Trafo* upd = fresh(&upd_s);
             if (upd_shift) {
 #pragma unroll
@@ -1605,7 +1628,9 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
             } else {
                 trafo_transform_to(*upd, R, Ru);
                 trafo_rotate_to(*upd, P, Pu);
+                if (push_next) push_step(Pu, step);
             }
+            if (push_next) push_move(Ru, step, bc.s_cdt, bc.rs_cdt);
         }
         x[i] = Ru[0];
         y[i] = Ru[1];
@@ -1640,6 +1665,8 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
     __syncthreads();
     if (threadIdx.x == 0) {
         StepState& s = *st;
+        s.pushed = push_next ? 1 : 0;
+        if (left_s > 0) s.left = left_s - 1;
         if (bc.sharded) {  // this rank's momentum sums; k_finish_psum completes after the exchange
             for (int k = 0; k < 3; ++k) put_limbs(s.xlimbs + 4 * k, ex[k]);
         } else {
