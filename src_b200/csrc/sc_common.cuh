@@ -239,39 +239,27 @@ SC_HD void quat_rotmat(const double* qin, double* M) {
     M[7] = 2 * (q[0] * q[1] + q[2] * q[3]);
     M[8] = 1 - 2 * (q[1] * q[1] + q[2] * q[2]);
 }
-// getQuaternion(u, ref); false for anti-parallel or null input.
-SC_HD bool get_quaternion(const double* uin, const double* refin, double* q) {
+// getQuaternion(u, (0, 0, 1)), false for an anti-parallel or null u: the products and sums with the components 0 and
+// 1 of the z axis left out (they change no bits but the sign of a zero), so
+// one square root and one quotient less in a chain that one thread runs.
+SC_HD bool get_quaternion_z(const double* uin, double* q) {
     const double tol = 1e-12;
-    double u[3] = {uin[0], uin[1], uin[2]}, ref[3] = {refin[0], refin[1], refin[2]};
-    double lu = sqrt(dot3(u, u)), lr = sqrt(dot3(ref, ref));
-    if (!(lu >= 1e-12) || !(lr >= 1e-12)) return false;
-    u[0] /= lu;
-    u[1] /= lu;
-    u[2] /= lu;
-    ref[0] /= lr;
-    ref[1] /= lr;
-    ref[2] /= lr;
-    double axis[3];
-    cross3(u, ref, axis);
-    double normAxis = sqrt(dot3(axis, axis));
+    const double lu = sqrt(dot3(uin, uin));
+    if (!(lu >= 1e-12)) return false;
+    const double u0 = uin[0] / lu, u1 = uin[1] / lu, u2 = uin[2] / lu;
+    const double normAxis = sqrt(u1 * u1 + u0 * u0);
     if (normAxis < tol) {
-        double d = dot3(u, ref) - 1.0;
-        if ((d < 0 ? -d : d) < tol) {
-            q[0] = 1.0;
-            q[1] = q[2] = q[3] = 0.0;
-            return true;
-        }
-        return false;
+        const double d = u2 - 1.0;
+        q[0] = 1.0;
+        q[1] = q[2] = q[3] = 0.0;
+        return (d < 0 ? -d : d) < tol;
     }
-    axis[0] /= normAxis;
-    axis[1] /= normAxis;
-    axis[2] /= normAxis;
-    double cosAngle = sqrt(0.5 * (1 + dot3(u, ref)));
-    double sinAngle = sqrt(1 - cosAngle * cosAngle);
+    const double cosAngle = sqrt(0.5 * (1 + u2));
+    const double sinAngle = sqrt(1 - cosAngle * cosAngle);
     q[0] = cosAngle;
-    q[1] = sinAngle * axis[0];
-    q[2] = sinAngle * axis[1];
-    q[3] = sinAngle * axis[2];
+    q[1] = sinAngle * (u1 / normAxis);
+    q[2] = sinAngle * (-u0 / normAxis);
+    q[3] = 0.0;
     return true;
 }
 
@@ -877,82 +865,118 @@ SC_HD void kick_r(double* P, const double* Ef, const double* Bf, double ke, doub
 }
 
 // ---------------------------------------------------------------- mesh
+// What derive_mesh reads, gathered by the caller (in shared memory on the
+// device) while the bounds are reduced, so that the one thread that derives
+// the mesh waits for no global load.
+struct MeshIn {
+    double bmin[3], bmax[3];  // beam-frame bounds
+    double psum_z, N;         // momentum sum and particles of the whole bunch
+    double dh, period, dT, Q;
+    int n[3];
+    int pz, binned;
+    unsigned gen;
+};
+
 // boundp (PartBunchBase.hpp:802-884) from the beam-frame bounds, then the
-// scalars of computeSelfFields (PartBunch.cpp:493-511, 541-547, 641).
-// Returns false when h <= 0.
-SC_HD_COLD bool derive_mesh(StepState& s, const BunchConst& bc) {
-    double rmin[3] = {s.bmin[0], s.bmin[1], s.bmin[2]};
-    double rmax[3] = {s.bmax[0], s.bmax[1], s.bmax[2]};
-    // a DC beam's z spans one period from the lowest particle, not enlarged
-    // (PartBunchBase.hpp:813-814, :840-843)
-    const int dims = bc.pz ? 2 : 3;
-    if (bc.pz) {
-        rmax[2] = rmin[2] + bc.period;
-        s.hr[2] = bc.period / (bc.n[2] - 1);
-        s.mesh_rmin[2] = rmin[2];
-        s.mesh_rmax[2] = rmax[2];
-    }
-    for (int i = 0; i < dims; ++i) {
-        double length = rmax[i] - rmin[i];
-        if (length < 0) length = -length;
-        if (length < 1e-10) {
-            rmax[i] += 1e-10;
-            rmin[i] -= 1e-10;
+// scalars of computeSelfFields (PartBunch.cpp:493-511, 541-547, 641) and the
+// charge of the scatter: Q *= dt; scatter; Q /= dt (PartBunch.cpp:493-495; the
+// energy-bin loop restores Q from its copy after every bin,
+// ParallelTTracker.cpp:570-576).  Values first, stores last: read back
+// through global memory they made a chain of 4000 cycles at the end of the
+// drift.  Returns false when h <= 0.
+SC_HD_COLD bool derive_mesh(StepState* st, const MeshIn* in) {
+    double rmin[3], rmax[3], hr[3], rhr[3], hs[3];
+    for (int i = 0; i < 3; ++i) {
+        rmin[i] = in->bmin[i];
+        rmax[i] = in->bmax[i];
+        // a DC beam's z spans one period from the lowest particle, not enlarged
+        // (PartBunchBase.hpp:813-814, :840-843)
+        if (i == 2 && in->pz) {
+            rmax[2] = rmin[2] + in->period;
+            hr[2] = in->period / (in->n[2] - 1);
         } else {
-            rmax[i] += bc.dh * length;
-            rmin[i] -= bc.dh * length;
+            double length = rmax[i] - rmin[i];
+            if (length < 0) length = -length;
+            const bool point = length < 1e-10;
+            const double grow = point ? 1e-10 : in->dh * length;
+            rmax[i] += grow;
+            rmin[i] -= grow;
+            hr[i] = (rmax[i] - rmin[i]) / (in->n[i] - 1);
         }
-        s.hr[i] = (rmax[i] - rmin[i]) / (bc.n[i] - 1);
-        s.mesh_rmin[i] = rmin[i];
-        s.mesh_rmax[i] = rmax[i];
+        rhr[i] = 1.0 / hr[i];
     }
-    bool ok = s.hr[0] * s.hr[1] * s.hr[2] > 0;
-    for (int i = 0; i < 3; ++i) s.origin[i] = rmin[i] - s.hr[i] / 2.0;
-    for (int i = 0; i < 3; ++i) s.rhr[i] = 1.0 / s.hr[i];
-    double gz = s.psum[2] / (double)bc.Ntot;
+    double gz = in->psum_z / in->N;
     gz *= gz;
     gz = sqrt(gz + 1.0);
+    hs[0] = hr[0] * 1.0;
+    hs[1] = hr[1] * 1.0;
+    hs[2] = hr[2] * 1.0;
+    hs[2] *= gz;
+    const double tmp2 = 1 / hs[0] * 1 / hs[1] * 1 / hs[2];
+    const double betaC = sqrt(gz * gz - 1.0) / gz / kC;
+    const double qdt = in->Q * in->dT;
+    const double q = qdt / in->dT;
+    StepState& s = *st;
+    for (int i = 0; i < 3; ++i) {
+        s.bmin[i] = in->bmin[i];
+        s.bmax[i] = in->bmax[i];
+        s.mesh_rmin[i] = rmin[i];
+        s.mesh_rmax[i] = rmax[i];
+        s.hr[i] = hr[i];
+        s.rhr[i] = rhr[i];
+        s.origin[i] = rmin[i] - hr[i] / 2.0;
+        s.hr_scaled[i] = hs[i];
+    }
     s.gammaz = gz;
-    s.hr_scaled[0] = s.hr[0] * 1.0;
-    s.hr_scaled[1] = s.hr[1] * 1.0;
-    s.hr_scaled[2] = s.hr[2] * 1.0;
-    s.hr_scaled[2] *= gz;
-    s.tmp2 = 1 / s.hr_scaled[0] * 1 / s.hr_scaled[1] * 1 / s.hr_scaled[2];
-    s.hvol = s.hr_scaled[0] * s.hr_scaled[1] * s.hr_scaled[2];
-    s.betaC = sqrt(gz * gz - 1.0) / gz / kC;
-    return ok;
+    s.tmp2 = tmp2;
+    s.hvol = hs[0] * hs[1] * hs[2];
+    s.betaC = betaC;
+    s.qdt = qdt;
+    if (!in->binned) s.Q = q;
+    const unsigned gen = in->gen + 1u;
+    s.gen = gen == 0u ? 1u : gen;
+    return hr[0] * hr[1] * hr[2] > 0;
 }
 
 // Beam-frame trafos of computeSpaceChargeFields (ParallelTTracker.cpp:550-554)
-// from the momentum sum and the path length.  Returns false for an
-// anti-parallel mean momentum.
-SC_HD_COLD bool derive_beam_frame(StepState& s, const BunchConst& bc) {
-    const double N = (double)bc.Ntot;
-    double pmean[3] = {s.psum[0] / N, s.psum[1] / N, s.psum[2] / N};
-    double zhat[3] = {0.0, 0.0, 1.0}, q[4];
-    bool ok = get_quaternion(pmean, zhat, q);
+// from the momentum sum (p0, p1, p2), the particle count and the path length.
+// Returns false for an anti-parallel mean momentum.
+SC_HD_COLD bool derive_beam_frame(StepState* s, double p0, double p1, double p2, double N, double path) {
+    const double pmean[3] = {p0 / N, p1 / N, p2 / N};
+    double q[4];
+    const bool ok = get_quaternion_z(pmean, q);
     if (!ok) {
         q[0] = 1.0;
         q[1] = q[2] = q[3] = 0.0;
     }
-    double qc[4] = {q[0], -q[1], -q[2], -q[3]};
-    double org[3] = {0.0, 0.0, s.path_length};
-    trafo_make(s.b2r, org, qc);
-    s.r2b = s.b2r;
-    trafo_invert(s.r2b);
+    const double qc[4] = {q[0], -q[1], -q[2], -q[3]};
+    const double org[3] = {0.0, 0.0, path};
+    Trafo b2r;
+    trafo_make(b2r, org, qc);
+    Trafo r2b = b2r;
+    trafo_invert(r2b);
+    s->psum[0] = p0;
+    s->psum[1] = p1;
+    s->psum[2] = p2;
+    s->b2r = b2r;
+    s->r2b = r2b;
     return ok;
 }
 
 // updateReferenceParticle + updateRefToLabCSTrafo (ParallelTTracker.cpp:1123-1212)
-// with the elements of the table and an optional uniform B_z.
+// with the elements of the table and an optional uniform B_z.  On copies of
+// the state, stored at the end.
 SC_HD bool advance_reference(StepState& s, const BunchConst& bc) {
-    s.ref_to_lab_step = s.ref_to_lab;  // the particles' external fields use the frame of the step's start
-    s.t_step = s.t;
-    s.t += bc.dT;
-    const double dt = s.t < bc.dT ? s.t : bc.dT;
+    double rr[3] = {s.ref_R[0], s.ref_R[1], s.ref_R[2]};
+    double rp[3] = {s.ref_P[0], s.ref_P[1], s.ref_P[2]};
+    Trafo ref_to_lab = s.ref_to_lab;
+    const double t0 = s.t;
+    const double path = s.path_length;
+    s.ref_to_lab_step = ref_to_lab;  // the particles' external fields use the frame of the step's start
+    s.t_step = t0;
+    const double t = t0 + bc.dT;
+    const double dt = t < bc.dT ? t : bc.dT;
     const double scaleFactor = kC * dt;
-    double* rr = s.ref_R;
-    double* rp = s.ref_P;
     double eref[3] = {0.0, 0.0, 0.0}, bref[3] = {0.0, 0.0, 0.0};
     for (int pass = 0; pass < 2; ++pass) {
         rr[0] /= scaleFactor;
@@ -969,31 +993,33 @@ SC_HD bool advance_reference(StepState& s, const BunchConst& bc) {
             // updateReferenceParticle (ParallelTTracker.cpp:1134-1155): the
             // elements' fields at the reference particle at t - dt / 2, then
             // the kick
-            add_external_fields(bc.sol, bc.nsol, s.ref_to_lab, rr, s.t - 0.5 * dt, eref, bref, true);
+            add_external_fields(bc.sol, bc.nsol, ref_to_lab, rr, t - 0.5 * dt, eref, bref, true);
             if (bc.bz_ext != 0.0) bref[2] += bc.bz_ext;
             kick_one(rp, eref, bref, dt, bc.mass, bc.charge);
         }
     }
-    s.path_length += sqrt(dot3(rr, rr));
-    double zhat[3] = {0.0, 0.0, 1.0}, qu[4];
-    bool ok = get_quaternion(rp, zhat, qu);
+    double qu[4];
+    bool ok = get_quaternion_z(rp, qu);
     if (!ok) {
         qu[0] = 1.0;
         qu[1] = qu[2] = qu[3] = 0.0;
     }
-    trafo_make(s.upd, rr, qu);
-    double v[3];
-    trafo_transform_to(s.upd, rr, v);
-    rr[0] = v[0];
-    rr[1] = v[1];
-    rr[2] = v[2];
-    trafo_rotate_to(s.upd, rp, v);
-    rp[0] = v[0];
-    rp[1] = v[1];
-    rp[2] = v[2];
-    Trafo inv = s.upd;
+    Trafo upd;
+    trafo_make(upd, rr, qu);
+    double vr[3], vp[3];
+    trafo_transform_to(upd, rr, vr);
+    trafo_rotate_to(upd, rp, vp);
+    Trafo inv = upd;
     trafo_invert(inv);
-    trafo_compose(s.ref_to_lab, inv);
+    trafo_compose(ref_to_lab, inv);
+    s.t = t;
+    s.path_length = path + sqrt(dot3(rr, rr));
+    s.upd = upd;
+    s.ref_to_lab = ref_to_lab;
+    for (int d = 0; d < 3; ++d) {
+        s.ref_R[d] = vr[d];
+        s.ref_P[d] = vp[d];
+    }
     return ok;
 }
 

@@ -83,7 +83,7 @@ __device__ __forceinline__ double ex_to_double(i128 x) {
     const unsigned long long hi = (unsigned long long)(m >> 64), lo = (unsigned long long)m;
     double r;
     if (hi == 0) {
-        r = __ull2double_rn(lo);
+        r = __ull2double_rn(lo) * 0x1p-72;
     } else {
         const int lz = __clzll(hi);
         const unsigned long long top = lz ? ((hi << lz) | (lo >> (64 - lz))) : hi;
@@ -91,9 +91,10 @@ __device__ __forceinline__ double ex_to_double(i128 x) {
         unsigned long long mant = top >> 11;
         const unsigned long long rem = top & 0x7ffull;
         if (rem > 0x400ull || (rem == 0x400ull && (rest != 0 || (mant & 1ull)))) mant += 1;
-        r = ldexp((double)mant, 75 - lz);
+        // mant 2^(75 - lz - kExFrac): a product with a power of two, exact
+        r = (double)mant * __longlong_as_double((long long)(1023 + 75 - kExFrac - lz) << 52);
     }
-    return ldexp(neg ? -r : r, -kExFrac);
+    return neg ? -r : r;
 }
 
 __device__ __forceinline__ i128 ex_shfl_down(i128 v, int off) {

@@ -69,14 +69,27 @@ __device__ __forceinline__ void load_mesh_consts(MeshConsts& m, const StepState*
 
 // ------------------------------------------------------------ reductions
 // Last-block-done: true in exactly one of the nblk blocks working on a bunch,
-// after every block's partials are visible.  The caller resets the ticket.
+// after every block's partials are visible: the barrier orders the block's
+// partials before thread 0's fence, the fence before its ticket.  (A fence by
+// every thread would make each wait for its own particle stores.)  The caller
+// resets the ticket.
 __device__ __forceinline__ bool last_block(unsigned* ticket, int nblk) {
     __shared__ bool am_last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) am_last = (atomicAdd(ticket, 1u) == (unsigned)nblk - 1u);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        am_last = (atomicAdd(ticket, 1u) == (unsigned)nblk - 1u);
+        __threadfence();
+    }
     __syncthreads();
     return am_last;
+}
+
+// Cooperative copy of a Trafo by threads first .. first + 15 of the block
+__device__ __forceinline__ void load_trafo(Trafo& dst, const Trafo* __restrict__ src, int first) {
+    static_assert(sizeof(Trafo) == 16 * sizeof(double), "16 words");
+    const int k = (int)threadIdx.x - first;
+    if (k >= 0 && k < 16) reinterpret_cast<double*>(&dst)[k] = reinterpret_cast<const double*>(src)[k];
 }
 
 // A 128-bit exact sum as four 32-bit chunks of its two's complement, each
@@ -127,10 +140,18 @@ __device__ __forceinline__ void final_sum_ex(const i128* partials, int nb, doubl
         i128 s[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) s[k] = 0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            const unsigned long long* q = reinterpret_cast<const unsigned long long*>(partials + (size_t)b * NV);
+        for (int b = threadIdx.x; b < nb; b += 2 * blockDim.x) {  // two rows in flight
+            const int b1 = b + blockDim.x;
+            const ulonglong2* q0 = reinterpret_cast<const ulonglong2*>(partials + (size_t)b * NV);
+            const ulonglong2* q1 = reinterpret_cast<const ulonglong2*>(partials + (size_t)(b1 < nb ? b1 : b) * NV);
+            ulonglong2 w0[NV], w1[NV];
 #pragma unroll
-            for (int k = 0; k < NV; ++k) s[k] += (i128)(((u128)__ldcg(q + 2 * k + 1) << 64) | __ldcg(q + 2 * k));
+            for (int k = 0; k < NV; ++k) w0[k] = __ldcg(q0 + k), w1[k] = __ldcg(q1 + k);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                s[k] += (i128)(((u128)w0[k].y << 64) | w0[k].x);
+                if (b1 < nb) s[k] += (i128)(((u128)w1[k].y << 64) | w1[k].x);
+            }
         }
         __shared__ i128 sm[NV][kWarps];
 #pragma unroll
@@ -172,9 +193,14 @@ __device__ __forceinline__ void final_min(const double* partials, int nb, double
     double s[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) s[k] = INFINITY;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    for (int b = threadIdx.x; b < nb; b += 2 * blockDim.x) {  // two rows in flight
+        const int b1 = b + blockDim.x < nb ? b + blockDim.x : b;
+        double w0[NV], w1[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) s[k] = fmin(s[k], __ldcg(partials + (size_t)b * NV + k));
+        for (int k = 0; k < NV; ++k) w0[k] = __ldcg(partials + (size_t)b * NV + k), w1[k] = __ldcg(partials + (size_t)b1 * NV + k);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) s[k] = fmin(s[k], fmin(w0[k], w1[k]));
+    }
     __shared__ double sm[NV][kWarps];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -251,7 +277,8 @@ __device__ __forceinline__ void reduce_state_body(const BunchConst& bc, const do
             st->psum[0] = tot[0];
             st->psum[1] = tot[1];
             st->psum[2] = tot[2];
-            if (init_frame && !derive_beam_frame(*st, bc)) atomicOr(&st->err, kFlagFrame);
+            if (init_frame && !derive_beam_frame(st, tot[0], tot[1], tot[2], (double)bc.Ntot, st->path_length))
+                atomicOr(&st->err, kFlagFrame);
         }
         *ticket = 0u;
     }
@@ -266,20 +293,22 @@ __global__ void __launch_bounds__(kThreads) k_reduce_state(BunchConst bc, const 
 }
 
 // ------------------------------------------------------------ drift + frame
-// The mesh of this step from the bounds in s.bmin / s.bmax, and the charge
-// of the scatter: Q *= dt; scatter; Q /= dt  (PartBunch.cpp:493-495); the
-// energy-bin loop restores Q from its copy after every bin
-// (ParallelTTracker.cpp:570-576).
-__device__ __forceinline__ void finish_mesh(StepState& s, const BunchConst& bc) {
-    if (!derive_mesh(s, bc)) atomicOr(&s.err, kFlagMesh);
-    s.qdt = s.Q * bc.dT;
-    if (!s.binned) s.Q = s.qdt / bc.dT;
-    s.gen += 1u;
-    if (s.gen == 0u) s.gen = 1u;
+// The inputs of this step's mesh but the bounds, from the state and the constants.
+__device__ __forceinline__ void load_mesh_in(MeshIn& m, const BunchConst& bc, const StepState* st) {
+    m.psum_z = st->psum[2];
+    m.Q = st->Q;
+    m.binned = st->binned;
+    m.gen = st->gen;
+    m.N = (double)bc.Ntot;
+    m.dh = bc.dh;
+    m.period = bc.period;
+    m.dT = bc.dT;
+    for (int k = 0; k < 3; ++k) m.n[k] = bc.n[k];
+    m.pz = bc.pz;
 }
 
-__device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6], StepState* st, double* partials,
-                                            unsigned* ticket, VB g);
+__device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6], StepState* st, MeshIn& mesh_in,
+                                            double* partials, unsigned* ticket, VB g);
 
 // Products and sums of the mixed form's FP64 steps, written as fused
 // multiply-adds (this file is compiled without contraction).
@@ -319,11 +348,11 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
                                            const double* __restrict__ py, const double* __restrict__ pz, StepState* st,
                                            double* partials, unsigned* ticket, VB g) {
     __shared__ Trafo r2b_s;
+    __shared__ MeshIn mesh_in_s;
     __shared__ int pushed_s;
-    if (threadIdx.x == 0) {
-        r2b_s = st->r2b;
-        pushed_s = st->pushed;
-    }
+    load_trafo(r2b_s, &st->r2b, 0);
+    if (threadIdx.x == 32) pushed_s = st->pushed;
+    if (threadIdx.x == 64) load_mesh_in(mesh_in_s, bc, st);
     __syncthreads();
     const bool push = DRIFT && pushed_s == 0;  // else the gather of the step before has pushed R
     double v[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};  // min x,y,z, -max x,y,z
@@ -373,14 +402,14 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
         v[4] = fmin(v[4], -R[1]);
         v[5] = fmin(v[5], -R[2]);
     }
-    bounds_tail(bc, v, st, partials, ticket, g);
+    bounds_tail(bc, v, st, mesh_in_s, partials, ticket, g);
 }
 
 // Block minimum of the per-thread bounds v (min x, y, z, -max x, y, z) into
 // partials[blk], then in the last block the bunch's bounds and its mesh
 // (sharded: this rank's bounds for the exchange).
-__device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6], StepState* st, double* partials,
-                                            unsigned* ticket, VB g) {
+__device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6], StepState* st, MeshIn& mesh_in,
+                                            double* partials, unsigned* ticket, VB g) {
     __shared__ double sm[6][kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -400,15 +429,14 @@ __device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6]
     final_min<6>(partials, g.nblk, tot);
     __syncthreads();
     if (threadIdx.x == 0) {
-        StepState& s = *st;
         if (bc.sharded) {  // this rank's bounds; k_finish_mesh completes after the exchange
-            for (int k = 0; k < 6; ++k) s.bnd6[k] = tot[k];
+            for (int k = 0; k < 6; ++k) st->bnd6[k] = tot[k];
         } else {
             for (int k = 0; k < 3; ++k) {
-                s.bmin[k] = tot[k];
-                s.bmax[k] = -tot[3 + k];
+                mesh_in.bmin[k] = tot[k];
+                mesh_in.bmax[k] = -tot[3 + k];
             }
-            finish_mesh(s, bc);
+            if (!derive_mesh(st, &mesh_in)) atomicOr(&st->err, kFlagMesh);
         }
         *ticket = 0u;
     }
@@ -1014,12 +1042,13 @@ __global__ void __launch_bounds__(kThreads) k_igf_G(int n0, int n1, int n2, cons
 // (bounds by min, exact sums as integer limbs), on one thread.
 __global__ void k_finish_mesh(BunchConst bc, StepState* st) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    StepState& s = *st;
+    MeshIn m;
+    load_mesh_in(m, bc, st);
     for (int k = 0; k < 3; ++k) {
-        s.bmin[k] = s.bnd6[k];
-        s.bmax[k] = -s.bnd6[3 + k];
+        m.bmin[k] = st->bnd6[k];
+        m.bmax[k] = -st->bnd6[3 + k];
     }
-    finish_mesh(s, bc);
+    if (!derive_mesh(st, &m)) atomicOr(&st->err, kFlagMesh);
 }
 
 // psum from the combined limbs; frame: the beam frame of the next step
@@ -1027,8 +1056,9 @@ __global__ void k_finish_mesh(BunchConst bc, StepState* st) {
 __global__ void k_finish_psum(BunchConst bc, StepState* st, int frame, int advance) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     StepState& s = *st;
-    for (int k = 0; k < 3; ++k) s.psum[k] = ex_to_double(get_limbs(s.xlimbs + 4 * k));
-    if (frame && !derive_beam_frame(s, bc)) atomicOr(&s.err, kFlagFrame);
+    double p[3];
+    for (int k = 0; k < 3; ++k) s.psum[k] = p[k] = ex_to_double(get_limbs(s.xlimbs + 4 * k));
+    if (frame && !derive_beam_frame(st, p[0], p[1], p[2], (double)bc.Ntot, s.path_length)) atomicOr(&s.err, kFlagFrame);
     if (advance) s.step += 1;
 }
 
@@ -1557,18 +1587,20 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
                                             double* sm = nullptr) {
     __shared__ Trafo b2r_s, upd_s;
     __shared__ MeshConsts ms;
-    __shared__ double betaC_s;
+    __shared__ double betaC_s, path_s;
     __shared__ int left_s;
     __shared__ unsigned long long big[3 * 4];
     __shared__ __align__(8) uint64_t bar[STAGED ? 2 * kWarps : 1];
+    // each thread loads a word or two: one trip to L2 before the loop
+    load_trafo(b2r_s, &st->b2r, 0);
+    load_trafo(upd_s, &st->upd, 32);
     load_mesh_consts(ms, st);
-    if (threadIdx.x < 12) big[threadIdx.x] = 0ull;
-    if (threadIdx.x == 0) {
-        b2r_s = st->b2r;
-        upd_s = st->upd;
-        betaC_s = st->betaC;
-        left_s = st->left;
-        if constexpr (STAGED) {
+    if (threadIdx.x >= 64 && threadIdx.x < 76) big[threadIdx.x - 64] = 0ull;
+    if (threadIdx.x == 96) betaC_s = st->betaC;
+    if (threadIdx.x == 97) left_s = st->left;
+    if (threadIdx.x == 98) path_s = st->path_length;
+    if constexpr (STAGED) {
+        if (threadIdx.x == 128) {
             for (int k = 0; k < 2 * kWarps; ++k) mbar_init(&bar[k], 1);
             mbar_fence_init();
         }
@@ -1670,10 +1702,7 @@ __device__ __forceinline__ void gather_body(const BunchConst& bc, double* __rest
         if (bc.sharded) {  // this rank's momentum sums; k_finish_psum completes after the exchange
             for (int k = 0; k < 3; ++k) put_limbs(s.xlimbs + 4 * k, ex[k]);
         } else {
-            s.psum[0] = tot[0];
-            s.psum[1] = tot[1];
-            s.psum[2] = tot[2];
-            if (!derive_beam_frame(s, bc)) atomicOr(&s.err, kFlagFrame);
+            if (!derive_beam_frame(st, tot[0], tot[1], tot[2], (double)bc.Ntot, path_s)) atomicOr(&s.err, kFlagFrame);
             s.step += 1;
         }
         *ticket = 0u;
