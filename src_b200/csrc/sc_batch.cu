@@ -203,7 +203,10 @@ int rebuild(scgpu_batch* b) {
     add_pass(3, kPassYInv);
     add_pass(3, kPassPlane);
     add_pass(3, kPassZC2R);
-    add_per_bunch(3, kBatchGrad, [&](const DevBunch& d) { return blocks_for(cells(d), 256, kCellGridCap); });
+    // blocks of 256 nodes of one plane
+    add_per_bunch(3, kBatchGrad, [](const DevBunch& d) {
+        return (int)std::min<long long>(((long long)d.bc.n[0] * d.bc.n[1] + 255) / 256 * d.bc.n[2], kCellGridCap);
+    });
     add_per_bunch(5, kBatchGather, [](const DevBunch& d) { return d.red_blocks; });
     if (nm > b->tab_cap) {
         if (b->d_tab) cudaFree(b->d_tab);

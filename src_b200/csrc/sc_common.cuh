@@ -96,6 +96,10 @@ struct StepState {
     int left;
     int pushed;
     int pad_;
+    // of the mesh, once per step for the kernels that use them per node
+    double gid[3];      // 0.5 / hr: the gradient's scale (UniformCartesian.hpp:2129-2203)
+    double gsc[2];      // gz / 1.0 (x, y) and 1.0 / (1.0 gz) (z): the boost of E (PartBunch.cpp:573-575)
+    double dep_unit;    // the deposit's unit of fixed-point charge, a power of two
     // sharded bunch: this rank's partial results, combined over the ranks
     // between kernels (bounds by min; exact sums as 32-bit chunks of the
     // 128-bit fixed point, summed as 64-bit integers)
@@ -161,6 +165,7 @@ struct BunchConst {
     // per-bunch constants of the pusher, evaluated in the reference's order
     double s_cdt;   // c * dT                      (PartBunchBase.hpp:481)
     double rs_cdt;  // RN(1 / (c * dT))
+    double rdT;     // RN(1 / dT), 0 below 2^-70 (div_rcp's limit)
     double ke;      // 0.5 * dT * charge * c / mass (BorisPusher.h:88)
     double ktn;     // 0.5 * dT * charge * c * c    (BorisPusher.h:99, numerator)
     // beamline elements with external fields (device table), none when nsol == 0
@@ -173,6 +178,7 @@ struct BunchConst {
 inline void bunch_constants(BunchConst& bc) {
     bc.s_cdt = kC * bc.dT;
     bc.rs_cdt = 1.0 / bc.s_cdt;
+    bc.rdT = bc.dT >= 0x1p-70 ? 1.0 / bc.dT : 0.0;
     bc.ke = 0.5 * bc.dT * bc.charge * kC / bc.mass;
     bc.ktn = 0.5 * bc.dT * bc.charge * kC * kC;
 }
@@ -865,6 +871,11 @@ SC_HD void kick_r(double* P, const double* Ef, const double* Bf, double ke, doub
 }
 
 // ---------------------------------------------------------------- mesh
+// Unit of the deposit's fixed point for charges of at most |qdt|: 2^(E - 52)
+// with 2^E > 2 |qdt| (sc_exact.cuh).
+constexpr int kFxFrac = 52;
+SC_HD double fx_unit(double qdt) { return ldexp(1.0, (qdt != 0.0 ? ilogb(qdt) + 2 : 0) - kFxFrac); }
+
 // What derive_mesh reads, gathered by the caller (in shared memory on the
 // device) while the bounds are reduced, so that the one thread that derives
 // the mesh waits for no global load.
@@ -926,7 +937,11 @@ SC_HD_COLD bool derive_mesh(StepState* st, const MeshIn* in) {
         s.rhr[i] = rhr[i];
         s.origin[i] = rmin[i] - hr[i] / 2.0;
         s.hr_scaled[i] = hs[i];
+        s.gid[i] = 0.5 / hr[i];
     }
+    s.gsc[0] = gz / 1.0;
+    s.gsc[1] = 1.0 / (1.0 * gz);
+    s.dep_unit = fx_unit(qdt);
     s.gammaz = gz;
     s.tmp2 = tmp2;
     s.hvol = hs[0] * hs[1] * hs[2];

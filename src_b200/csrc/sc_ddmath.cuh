@@ -287,9 +287,14 @@ SC_DDM_HD double rcp_approx(double d) {
 // tail is below 2^-18.5 hi; the largest seen over 2e7 arguments is 2^-67.8).
 constexpr double kAtanQuickEps = 0x1p-66;
 SC_DDM_HD hilo atan_hilo(double a) {
-    const bool inv = a > 1.0;
+    const bool inv = (uint32_t)(bits_of(a) >> 32) >= 0x3ff00000u;  // a >= 1, on the integer units
     const float f = (float)a;
+    // a float quotient a few ulp off may pick the neighbour of round(128 / a)
+#ifdef __CUDA_ARCH__
+    const int j = __float2int_rn(inv ? __fdividef(128.0f, f) : 128.0f * f);
+#else
     const int j = (int)rintf(inv ? 128.0f / f : 128.0f * f);
+#endif
     const int row = inv ? j + 129 : j;
     const double th0 = kAtanQ[row][0], tl0 = kAtanQ[row][1];
     // j / 128: 2^45 + j / 128 has j in its low word
@@ -315,21 +320,27 @@ SC_DDM_HD hilo atan_hilo(double a) {
 SC_DDM_HD bool atan_quick(double x, double& out) {
     const hilo v = atan_hilo(fabs(x));
     const double r = v.hi + fma(v.hi, kAtanQuickEps, v.lo);
-    out = x < 0.0 ? -r : r;
+    out = copysign(r, x);
     return r == v.hi + fma(v.hi, -kAtanQuickEps, v.lo);
 }
 
 // Correctly rounded log and atan (the quick phase, else the full evaluation).
+// The ranges are tested on the high word: x positive, normal and finite (log
+// 1 is undecided in the quick phase); 2^-30 <= |x| < 2^30.
+SC_DDM_HD bool log_range(double x) { return (uint32_t)(bits_of(x) >> 32) - 0x00100000u < 0x7fe00000u; }
+SC_DDM_HD bool atan_range(double x) {
+    return ((uint32_t)(bits_of(x) >> 32) & 0x7fffffffu) - 0x3e100000u < 0x41d00000u - 0x3e100000u;
+}
+
 SC_DDM_HD double log_dd(double x) {
     double r;
-    if (x >= 2.2250738585072014e-308 && x <= 1.7976931348623157e308 && x != 1.0 && log_quick(x, r)) return r;
+    if (log_range(x) && log_quick(x, r)) return r;
     return log_dd_full(x);
 }
 
 SC_DDM_HD double atan_dd(double x) {
-    const double a = fabs(x);
     double r;
-    if (a >= 9.3132257461547852e-10 && a <= 1073741824.0 && atan_quick(x, r)) return r;
+    if (atan_range(x) && atan_quick(x, r)) return r;
     return atan_dd_full(x);
 }
 
@@ -337,18 +348,16 @@ SC_DDM_HD double atan_dd(double x) {
 // rounded once, within 0.5001 ulp for log and atan of the arguments the
 // quick phases take (log next to 1 within an ulp).
 SC_DDM_HD double log_fast(double x) {
-    if (!(x >= 2.2250738585072014e-308 && x <= 1.7976931348623157e308)) return log(x);
+    if (!log_range(x)) return log(x);
     bool exact;
     const hilo v = log_hilo(x, exact);
     return v.hi + v.lo;
 }
 
 SC_DDM_HD double atan_fast(double x) {
-    const double a = fabs(x);
-    if (!(a >= 9.3132257461547852e-10 && a <= 1073741824.0)) return atan(x);
-    const hilo v = atan_hilo(a);
-    const double r = v.hi + v.lo;
-    return x < 0.0 ? -r : r;
+    if (!atan_range(x)) return atan(x);
+    const hilo v = atan_hilo(fabs(x));
+    return copysign(v.hi + v.lo, x);
 }
 
 }  // namespace ddm

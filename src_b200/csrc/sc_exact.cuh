@@ -10,6 +10,8 @@
 
 #include <cstdint>
 
+#include "sc_common.cuh"
+
 namespace sc {
 
 using i128 = __int128;
@@ -110,10 +112,6 @@ __device__ __forceinline__ i128 ex_shfl_down(i128 v, int off) {
 // the sums are integer additions, exact, so any order gives the same total,
 // which is rounded to a double once.  The rounding of t is at most 2^-52 of
 // one particle's charge.
-constexpr int kFxFrac = 52;
-
-__device__ __forceinline__ int fx_exponent(double qdt) { return qdt != 0.0 ? ilogb(qdt) + 2 : 0; }
-
 // correctly rounded double of the 128-bit accumulator (lo, hi), times unit
 __device__ __forceinline__ double acc_to_double(unsigned long long lo, unsigned long long hi, double unit) {
     const long long shi = (long long)hi;
@@ -130,17 +128,20 @@ __device__ __forceinline__ double acc_to_double(unsigned long long lo, unsigned 
     unsigned long long mant = top >> 11;
     const unsigned long long rem = top & 0x7ffull;
     if (rem > 0x400ull || (rem == 0x400ull && (rest != 0 || (mant & 1ull)))) mant += 1;
-    const double r = ldexp((double)mant, 75 - lz);
+    const double r = (double)mant * __longlong_as_double((long long)(1023 + 75 - lz) << 52);  // mant 2^(75 - lz)
     return (neg ? -r : r) * unit;
 }
 
 // The charge density of one node from its accumulator (L, H) = H 2^32 + L:
 // (exact node sum) / dT * tmp2 (PartBunch.cpp:496, :510-511).  Only a
-// product and a quotient: no contraction can change its rounding.
-__device__ __forceinline__ double node_density(ulonglong2 a, double unit, double dT, double tmp2) {
-    const i128 w = (i128)(long long)a.y * (i128)4294967296 + (i128)a.x;
+// product and a quotient: no contraction can change its rounding.  rdT: RN(1
+// / dT), or 0 to divide (dT below 2^-70, where div_rcp does not hold); an
+// empty node skips the quotient.
+__device__ __forceinline__ double node_density(ulonglong2 a, double unit, double dT, double rdT, double tmp2) {
+    if ((a.x | a.y) == 0ull) return 0.0 * tmp2;
+    const i128 w = ((i128)(long long)a.y << 32) + (i128)a.x;
     double s = acc_to_double((unsigned long long)w, (unsigned long long)(w >> 64), unit);
-    s /= dT;
+    s = rdT != 0.0 ? div_rcp(s, dT, rdT) : s / dT;
     s *= tmp2;
     return s;
 }

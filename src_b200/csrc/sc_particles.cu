@@ -20,6 +20,7 @@
 //                        next step's first half drift
 //   k_gather_staged      the same with the particle state streamed through shared
 //                        memory by bulk copies (cp.async.bulk, mbarrier), the default
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -55,6 +56,25 @@ struct VB {
     int blk, nblk;
 };
 __device__ __forceinline__ VB vb_grid() { return VB{(int)blockIdx.x, (int)gridDim.x}; }
+
+// f(i, j, k, c) on every node c = i + n0 (j + n1 k) of a grid: a block takes
+// blockDim.x nodes of one plane at a time, so the plane index is the block's
+// and a thread divides once (three quotients and remainders per node were a
+// third of the gradient's instructions).
+template <typename F>
+__device__ __forceinline__ void for_plane_nodes(int n0, int n1, int n2, VB g, F&& f) {
+    const int nxy = n0 * n1;
+    const int chunks = (nxy + (int)blockDim.x - 1) / (int)blockDim.x;
+    for (int b = g.blk; b < chunks * n2; b += g.nblk) {
+        const int k = b / chunks;
+        const int p = (b - k * chunks) * (int)blockDim.x + (int)threadIdx.x;
+        if (p >= nxy) continue;
+        const int j = p / n0;
+        f(p - j * n0, j, k, k * nxy + p);
+    }
+}
+// its blocks of kThreads
+inline long long plane_blocks(long long n0, long long n1, long long n2) { return (n0 * n1 + kThreads - 1) / kThreads * n2; }
 
 struct MeshConsts {
     double hr[3], rhr[3], org[3];
@@ -587,7 +607,7 @@ __device__ __forceinline__ void cic_charge(const double* d, double q, double* v)
     v[7] = d[0] * d[1] * d[2] * q;
 }
 
-// Exact sums of the scattered charges (kFxFrac, fx_exponent, node_density in
+// Exact sums of the scattered charges (kFxFrac, fx_unit, node_density in
 // sc_exact.cuh).
 
 // A fixed-point charge t = rint(v) (|t| < 2^51; the conversion rounds half
@@ -650,7 +670,7 @@ __device__ __forceinline__ void deposit_body(const BunchConst& bc, const double*
     load_mesh_consts(ms, st);
     if (threadIdx.x == 0) {
         qdt_s = st->qdt;
-        to_int_s = ldexp(1.0, kFxFrac - fx_exponent(st->qdt));
+        to_int_s = 1.0 / st->dep_unit;  // a power of two
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -743,7 +763,7 @@ __device__ __forceinline__ void deposit_pairs_body(const BunchConst& bc, const d
     load_mesh_consts(ms, st);
     if (threadIdx.x == 0) {
         qdt_s = st->qdt;
-        to_int_s = ldexp(1.0, kFxFrac - fx_exponent(st->qdt));
+        to_int_s = 1.0 / st->dep_unit;  // a power of two
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -955,10 +975,11 @@ __device__ __forceinline__ void assemble_body(const BunchConst& bc, const StepSt
                                               unsigned long long* __restrict__ acc, T* __restrict__ rho, VB g,
                                               bool weights) {
     const int M = bc.n[0] * bc.n[1] * bc.n[2];
-    const double dT = bc.dT, tmp2 = st->tmp2;
-    const double unit = weights ? ldexp(st->qdt, -kWeightFrac) : ldexp(1.0, fx_exponent(st->qdt) - kFxFrac);
+    const double dT = bc.dT, rdT = bc.rdT, tmp2 = st->tmp2;
+    const double unit = weights ? st->qdt * 0x1p-26 : st->dep_unit;
+    static_assert(kWeightFrac == 26, "the weights' unit");
     for (int c = g.blk * blockDim.x + threadIdx.x; c < M; c += g.nblk * blockDim.x) {
-        const double s = node_density(reinterpret_cast<const ulonglong2*>(acc)[c], unit, dT, tmp2);
+        const double s = node_density(reinterpret_cast<const ulonglong2*>(acc)[c], unit, dT, rdT, tmp2);
         rho[c] = (T)s;
         reinterpret_cast<ulonglong2*>(acc)[c] = make_ulonglong2(0ull, 0ull);
     }
@@ -1016,7 +1037,7 @@ __device__ __forceinline__ void igf_tmp_body(int n0, int n1, int n2, const StepS
     }
 }
 template <bool CR = true>
-__global__ void __launch_bounds__(kThreads) k_igf_tmp(int n0, int n1, int n2, const StepState* __restrict__ st,
+__global__ void __launch_bounds__(kThreads, 5) k_igf_tmp(int n0, int n1, int n2, const StepState* __restrict__ st,
                                                       double* __restrict__ tmp) {
     igf_tmp_body<CR>(n0, n1, n2, st, tmp, vb_grid());
 }
@@ -1077,7 +1098,7 @@ __global__ void k_finish_stats(StepState* st) {
 // z = k hz - hz/2 + zshift (tmpgreen), set 1 at z = k hz - hz/2 + zshift - n2 hz
 // (grn2), k in [0, n2+1]; x, y as in the unshifted function.  hz and zshift
 // are the bin's (st->hr_scaled, st->zshift).
-__global__ void __launch_bounds__(kThreads) k_igf_tmp_img(int n0, int n1, int n2, const StepState* __restrict__ st,
+__global__ void __launch_bounds__(kThreads, 5) k_igf_tmp_img(int n0, int n1, int n2, const StepState* __restrict__ st,
                                                           double* __restrict__ tmp) {
     const int t0 = n0 + 2, t1 = n1 + 2, t2 = n2 + 2;
     const int T3 = t0 * t1 * t2;
@@ -1213,6 +1234,10 @@ __global__ void __launch_bounds__(kThreads) k_bin_gammas(BunchConst bc, const do
             o.origin[d] = st->origin[d];
         }
         o.qdt = st->qdt;
+        o.dep_unit = st->dep_unit;
+        for (int d = 0; d < 3; ++d) o.gid[d] = st->gid[d];
+        o.gsc[0] = gz / 1.0;
+        o.gsc[1] = 1.0 / (1.0 * gz);
         const double scaleFactor = 1;
         o.gammaz = gz;
         o.bin_count = cnt;
@@ -1228,23 +1253,30 @@ __global__ void __launch_bounds__(kThreads) k_bin_gammas(BunchConst bc, const do
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
-// -grad phi (UniformCartesian.hpp:2129-2203, scaled by the bin's (g, g, 1/g),
-// PartBunch.cpp:199-200) of one node of a potential.
+// -grad phi (UniformCartesian.hpp:2129-2203), scaled by (g, g, 1/g)
+// (PartBunch.cpp:199-200, :573-575), of one node of a potential: the scales are
+// st->gid and st->gsc.
+struct GradConsts {
+    int n[3], stride[3];
+    double id[3], sc[3];
+    __device__ __forceinline__ GradConsts(const BunchConst& bc, const StepState* __restrict__ st)
+        : n{bc.n[0], bc.n[1], bc.n[2]}, stride{1, bc.n[0], bc.n[0] * bc.n[1]}, id{st->gid[0], st->gid[1], st->gid[2]},
+          sc{st->gsc[0], st->gsc[0], st->gsc[1]} {}
+};
 __device__ __forceinline__ void neg_grad_scaled(const double* __restrict__ phi, int c, const int (&idx)[3],
-                                                const int (&n)[3], const int (&stv)[3], const double (&id)[3],
-                                                const double (&sc)[3], double (&e)[3]) {
+                                                const GradConsts& q, double (&e)[3]) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double* f = phi + c;
-        const int s = stv[d];
+        const int s = q.stride[d];
         double g;
         if (idx[d] == 0)
-            g = id[d] * (-1.0 * f[2 * s] + 4.0 * f[s] - 3.0 * f[0]);
-        else if (idx[d] == n[d] - 1)
-            g = id[d] * (1.0 * f[-2 * s] - 4.0 * f[-s] + 3.0 * f[0]);
+            g = q.id[d] * (-1.0 * f[2 * s] + 4.0 * f[s] - 3.0 * f[0]);
+        else if (idx[d] == q.n[d] - 1)
+            g = q.id[d] * (1.0 * f[-2 * s] - 4.0 * f[-s] + 3.0 * f[0]);
         else
-            g = id[d] * (f[s] - f[-s]);
-        e[d] = (-g) * sc[d];
+            g = q.id[d] * (f[s] - f[-s]);
+        e[d] = (-g) * q.sc[d];
     }
 }
 
@@ -1255,19 +1287,13 @@ __device__ __forceinline__ void neg_grad_scaled(const double* __restrict__ phi, 
 __global__ void __launch_bounds__(kThreads, 4) k_grad_acc(BunchConst bc, const StepState* __restrict__ st,
                                                        const double* __restrict__ phi,
                                                        const double* __restrict__ phi_img, double* __restrict__ F8) {
-    const int n[3] = {bc.n[0], bc.n[1], bc.n[2]};
-    const int M = n[0] * n[1] * n[2];
-    const int stv[3] = {1, n[0], n[0] * n[1]};
-    const double h[3] = {st->hr[0], st->hr[1], st->hr[2]};
-    const double id[3] = {0.5 / h[0], 0.5 / h[1], 0.5 / h[2]};
-    const double gz = st->gammaz;
-    const double sc[3] = {gz / 1.0, gz / 1.0, 1.0 / (1.0 * gz)};
+    const GradConsts q(bc, st);
     const double betaC = st->betaC;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < M; c += gridDim.x * blockDim.x) {
-        const int idx[3] = {c % n[0], (c / n[0]) % n[1], c / (n[0] * n[1])};
+    for_plane_nodes(q.n[0], q.n[1], q.n[2], vb_grid(), [&](int i, int j, int k, int c) {
+        const int idx[3] = {i, j, k};
         double e[3], ei[3];
-        neg_grad_scaled(phi, c, idx, n, stv, id, sc, e);
-        neg_grad_scaled(phi_img, c, idx, n, stv, id, sc, ei);
+        neg_grad_scaled(phi, c, idx, q, e);
+        neg_grad_scaled(phi_img, c, idx, q, ei);
         double* o = F8 + 8 * (size_t)c;
         double2 exy = *reinterpret_cast<const double2*>(o);
         double2 ez = *reinterpret_cast<const double2*>(o + 2);
@@ -1285,7 +1311,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_grad_acc(BunchConst bc, const S
         *reinterpret_cast<double2*>(o) = exy;
         *reinterpret_cast<double2*>(o + 2) = ez;
         *reinterpret_cast<double2*>(o + 4) = bxy;
-    }
+    });
 }
 
 // get_bounds of the particle positions (PartBunchBase.hpp:1178-1219) for the
@@ -1360,34 +1386,19 @@ __global__ void __launch_bounds__(kThreads) k_permute_i32(const uint32_t* __rest
 template <typename T>
 __device__ __forceinline__ void grad_body(const BunchConst& bc, const StepState* __restrict__ st,
                                           const double* __restrict__ phi, T* __restrict__ E4, VB g) {
-    const int n[3] = {bc.n[0], bc.n[1], bc.n[2]};
-    const int M = n[0] * n[1] * n[2];
-    const int stv[3] = {1, n[0], n[0] * n[1]};
-    const double h[3] = {st->hr[0], st->hr[1], st->hr[2]};
-    const double id[3] = {0.5 / h[0], 0.5 / h[1], 0.5 / h[2]};
-    const double gz = st->gammaz;
-    const double sc[3] = {gz / 1.0, gz / 1.0, 1.0 / (1.0 * gz)};
-    for (int c = g.blk * blockDim.x + threadIdx.x; c < M; c += g.nblk * blockDim.x) {
-        const int idx[3] = {c % n[0], (c / n[0]) % n[1], c / (n[0] * n[1])};
+    const GradConsts q(bc, st);
+    for_plane_nodes(q.n[0], q.n[1], q.n[2], g, [&](int i, int j, int k, int c) {
+        const int idx[3] = {i, j, k};
         double e[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double* f = phi + c;
-            const int s = stv[d];
-            double g;
-            if (idx[d] == 0)
-                g = id[d] * (-1.0 * (double)f[2 * s] + 4.0 * (double)f[s] - 3.0 * (double)f[0]);
-            else if (idx[d] == n[d] - 1)
-                g = id[d] * (1.0 * (double)f[-2 * s] - 4.0 * (double)f[-s] + 3.0 * (double)f[0]);
-            else
-                g = id[d] * ((double)f[s] - (double)f[-s]);
-            e[d] = (-g) * sc[d];
+        neg_grad_scaled(phi, c, idx, q, e);
+        T* o = E4 + 4 * (size_t)c;
+        if constexpr (sizeof(T) == sizeof(double)) {
+            reinterpret_cast<double2*>(o)[0] = make_double2(e[0], e[1]);
+            reinterpret_cast<double2*>(o)[1] = make_double2(e[2], 0.0);
+        } else {
+            *reinterpret_cast<float4*>(o) = make_float4((float)e[0], (float)e[1], (float)e[2], 0.0f);
         }
-        E4[4 * (size_t)c + 0] = (T)e[0];
-        E4[4 * (size_t)c + 1] = (T)e[1];
-        E4[4 * (size_t)c + 2] = (T)e[2];
-        E4[4 * (size_t)c + 3] = (T)0;
-    }
+    });
 }
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_grad(BunchConst bc, const StepState* __restrict__ st,
@@ -1871,6 +1882,8 @@ __global__ void __launch_bounds__(kThreads) k_convert(const TI* __restrict__ in,
         out[i] = (TO)in[i];
 }
 
+constexpr int kGridCap = 148 * 16;  // blocks of a grid kernel; the rest loops
+
 inline int grid_for(long long work, int cap) {
     long long g = (work + kThreads - 1) / kThreads;
     if (g < 1) g = 1;
@@ -1921,7 +1934,7 @@ __global__ void k_advance_batch(const DevBunch* __restrict__ tab, const int4* __
     advance_reference_body(d.bc, d.st, VB{w.y, w.w});
 }
 
-__global__ void __launch_bounds__(kThreads) k_igf_tmp_batch(const DevBunch* __restrict__ tab, const int4* __restrict__ work, int nitems) {
+__global__ void __launch_bounds__(kThreads, 5) k_igf_tmp_batch(const DevBunch* __restrict__ tab, const int4* __restrict__ work, int nitems) {
     const int4 w = resolve_block(work, nitems);
     const DevBunch& d = tab[w.x];
     if (d.precision == 0)
@@ -2114,12 +2127,8 @@ void launch_assemble_rho(const DevBunch& b, cudaStream_t s) {
 void launch_igf(const DevBunch& b, const double* hr_host, cudaStream_t s) {
     (void)hr_host;
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
-    const long long T3 = (long long)(n0 + 2) * (n1 + 2) * (n2 + 2);
     const long long G3 = (long long)(n0 + 1) * (n1 + 1) * (n2 + 1);
-    if (b.precision == 0)
-        k_igf_tmp<true><<<grid_for(T3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
-    else
-        k_igf_tmp<false><<<grid_for(T3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
+    launch_igf_tmp(b, s);
     k_igf_G<<<grid_for(G3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.gtmp, b.gline);
 }
 
@@ -2127,16 +2136,15 @@ void launch_igf(const DevBunch& b, const double* hr_host, cudaStream_t s) {
 // from it inside its first cosine transform.
 void launch_igf_tmp(const DevBunch& b, cudaStream_t s) {
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
-    const long long T3 = (long long)(n0 + 2) * (n1 + 2) * (n2 + 2);
+    const int g = grid_for((long long)(n0 + 2) * (n1 + 2) * (n2 + 2), kGridCap);
     if (b.precision == 0)
-        k_igf_tmp<true><<<grid_for(T3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
+        k_igf_tmp<true><<<g, kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
     else
-        k_igf_tmp<false><<<grid_for(T3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
+        k_igf_tmp<false><<<g, kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp);
 }
 
 void launch_grad(const DevBunch& b, cudaStream_t s) {
-    const long long M = (long long)b.bc.n[0] * b.bc.n[1] * b.bc.n[2];
-    const int g = grid_for(M, 148 * 16);
+    const int g = (int)std::min<long long>(plane_blocks(b.bc.n[0], b.bc.n[1], b.bc.n[2]), kGridCap);
     if (b.precision == 0)
         k_grad<double><<<g, kThreads, 0, s>>>(b.bc, b.st, b.phi, (double*)b.E4);
     else
@@ -2198,8 +2206,7 @@ void launch_deposit_bins(const DevBunch& b, cudaStream_t s) {
 }
 
 void launch_grad_acc(const DevBunch& v, const double* phi_img, cudaStream_t s) {
-    const long long M = (long long)v.bc.n[0] * v.bc.n[1] * v.bc.n[2];
-    const int g = grid_for(M, 148 * 16);
+    const int g = (int)std::min<long long>(plane_blocks(v.bc.n[0], v.bc.n[1], v.bc.n[2]), kGridCap);
     k_grad_acc<<<g, kThreads, 0, s>>>(v.bc, v.st, v.phi, phi_img, v.F8);
 }
 
@@ -2233,9 +2240,9 @@ void launch_permute_bins(const DevBunch& b, cudaStream_t s) {
 
 void launch_igf_image(const DevBunch& b, cudaStream_t s) {
     const int n0 = b.bc.n[0], n1 = b.bc.n[1], n2 = b.bc.n[2];
-    const long long T3 = (long long)(n0 + 2) * (n1 + 2) * (n2 + 2);
     const long long GI = (long long)(n0 + 1) * (n1 + 1) * (2 * n2);
-    k_igf_tmp_img<<<grid_for(2 * T3, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp_img);
+    const long long T3 = (long long)(n0 + 2) * (n1 + 2) * (n2 + 2);
+    k_igf_tmp_img<<<grid_for(2 * T3, kGridCap), kThreads, 0, s>>>(n0, n1, n2, b.st, b.gtmp_img);
     k_igf_G_img<<<grid_for(GI, 148 * 16), kThreads, 0, s>>>(n0, n1, n2, b.gtmp_img, b.gimg);
 }
 
