@@ -266,6 +266,8 @@ DevBunch bin_view(const scgpu_ctx* c, int k) {
     return v;
 }
 
+void enqueue_reorder_beside(scgpu_ctx* c, cudaEvent_t after);
+
 // The energy-bin loop of computeSpaceChargeFields (ParallelTTracker.cpp:567-578)
 // once the drift kernel has set this step's mesh: calcGammas, one deposit pass
 // for all active bins, then per bin the charge density, the bin's own
@@ -273,12 +275,16 @@ DevBunch bin_view(const scgpu_ctx* c, int k) {
 // each field added into F8.  The Green's functions of a bin depend on its
 // gamma only, so they run on the side stream, at most two bins ahead of the
 // main stream's convolutions (two sets of spectra).
-void enqueue_bins_fields(scgpu_ctx* c, cudaStream_t s) {
+void enqueue_bins_fields(scgpu_ctx* c, bool reorder, cudaStream_t s) {
     DevBunch& b = c->b;
     const long long M = mesh_cells(b);
     launch_bin_gammas(b, s);
     cudaMemsetAsync(b.F8, 0, (size_t)M * 8 * sizeof(double), s);
     launch_deposit_bins(b, s);
+    if (reorder) {
+        cudaEventRecord(c->ev_dep, s);
+        enqueue_reorder_beside(c, c->ev_dep);
+    }
     if (b.nactive <= 0) return;
     cudaEventRecord(c->ev_fork, s);
     cudaStreamWaitEvent(c->side, c->ev_fork, 0);
@@ -370,7 +376,15 @@ void enqueue_reorder(scgpu_ctx* c, cudaStream_t s) {
     launch_sort(b, s);
     launch_reorder(b, s);
     if (b.nbins > 0) launch_permute_bins(b, s);
-    cudaMemsetAsync(b.hist, 0, (size_t)b.bc.n[0] * b.bc.n[1] * b.bc.n[2] * sizeof(int), s);
+}
+
+// The reorder of a step beside its solve: the particles rest between the
+// deposit and the gather, so it runs on the reference particle's stream from
+// the event `after` (the deposit) and joins with it before the gather.
+void enqueue_reorder_beside(scgpu_ctx* c, cudaEvent_t after) {
+    cudaStreamWaitEvent(c->ref, after, 0);
+    enqueue_reorder(c, c->ref);
+    cudaEventRecord(c->ev_ref, c->ref);
 }
 
 // The Green's function and its spectrum (open or periodic z), shared by the
@@ -387,8 +401,9 @@ void enqueue_green(scgpu_ctx* c, cudaStream_t s) {
 
 // one ParallelTTracker step on the context's stream
 //   ref:  reference-particle update (needs only the tracker state; joins
-//         before the gather, which applies its frame change)
-//   main: drift -> deposit -> assemble [-> reorder] -> FFT A, B
+//         before the gather, which applies its frame change), then on a
+//         reorder step, after the deposit, the particles' cell order
+//   main: drift -> deposit -> assemble -> FFT A, B
 //   side: (after the drift's mesh) Green's function, its spectrum
 //   main: (join side) FFT C, D, E -> grad -> (join ref) gather/kick/push
 // The branches write disjoint StepState fields.
@@ -409,10 +424,13 @@ void enqueue_step(scgpu_ctx* c, bool stats, bool reorder, cudaStream_t s) {
     enqueue_green(c, c->side);
     cudaEventRecord(c->ev_join, c->side);
     launch_deposit(b, s);
+    if (reorder) {
+        cudaEventRecord(c->ev_dep, s);
+        enqueue_reorder_beside(c, c->ev_dep);
+    }
     if (shard)  // the charge of all shards: exact integer node sums
         exchange(c, b.nacc, 2 * mesh_cells(b), SCGPU_EXCHANGE_SUM_U64, s);
     launch_assemble_rho(b, s);
-    if (reorder) enqueue_reorder(c, s);
     launch_convolution_part(b, kConvSelfField, kConvForwardPart, s);
     cudaStreamWaitEvent(s, c->ev_join, 0);
     launch_convolution_part(b, kConvSelfField, kConvRestPart, s);
@@ -437,8 +455,7 @@ void enqueue_step_binned(scgpu_ctx* c, bool stats, bool reorder, cudaStream_t s)
     launch_advance_reference(b, c->ref);
     cudaEventRecord(c->ev_ref, c->ref);
     launch_drift_to_beam(b, true, s);
-    enqueue_bins_fields(c, s);
-    if (reorder) enqueue_reorder(c, s);
+    enqueue_bins_fields(c, reorder, s);
     cudaStreamWaitEvent(s, c->ev_ref, 0);
     launch_gather_kick_push_bins(b, stats, s);
 }
@@ -640,6 +657,7 @@ int scgpu_create(scgpu_ctx** out, const scgpu_solver_params* p, int device) {
     cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&c->ev_ref, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&c->ev_dep, cudaEventDisableTiming);
     cudaEventCreate(&c->ev_t0);
     cudaEventCreate(&c->ev_t1);
     cudaMemsetAsync(b.nacc, 0, M * 2 * sizeof(unsigned long long), c->own);
@@ -680,6 +698,7 @@ void scgpu_destroy(scgpu_ctx* c) {
     if (c->ev_t1) cudaEventDestroy(c->ev_t1);
     if (c->ev_start) cudaEventDestroy(c->ev_start);
     if (c->ev_ref) cudaEventDestroy(c->ev_ref);
+    if (c->ev_dep) cudaEventDestroy(c->ev_dep);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ref) cudaStreamDestroy(c->ref);
     if (c->own) cudaStreamDestroy(c->own);
@@ -1270,7 +1289,7 @@ int scgpu_compute_self_fields_binned(scgpu_ctx* c, long long n, const double* R,
     STAGE("reduce_state");
     launch_drift_to_beam(b, false, s);
     STAGE("bounds");
-    enqueue_bins_fields(c, s);
+    enqueue_bins_fields(c, false, s);
     STAGE("bins");
     launch_gather_fields_bins(b, s);
     STAGE("gather");

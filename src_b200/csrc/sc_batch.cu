@@ -8,8 +8,9 @@
 // passes are grouped by the transform length of their axis, since the length
 // is a template constant of the kernels.  The step order is the single-bunch one (sc_api.cu enqueue_step):
 //
-//   ref:  reference-particle updates (joined before the gather)
-//   main: drift -> deposit -> assemble [-> cell reorder] -> FFT A, B
+//   ref:  reference-particle updates, [the cell reorder after the deposit]
+//         (joined before the gather)
+//   main: drift -> deposit -> assemble -> FFT A, B
 //   side: Green's function (antiderivative, 8-corner G, three DCT passes)
 //   main: (join side) FFT C, D, E -> grad -> (join ref) gather/kick/push
 //
@@ -68,7 +69,7 @@ struct scgpu_batch {
     std::vector<scgpu_ctx*> slots;
     std::vector<int> members;   // occupied slots in table order
     cudaStream_t stream = nullptr, side = nullptr, ref = nullptr;
-    cudaEvent_t ev_start = nullptr, ev_ref = nullptr;
+    cudaEvent_t ev_start = nullptr, ev_ref = nullptr, ev_dep = nullptr;
     // Uploads and downloads of the bunches run here, at the highest stream
     // priority, so that a bunch joining during a long batched round gets SMs
     // as soon as blocks of the round retire instead of waiting for the round.
@@ -255,8 +256,12 @@ void enqueue_step(scgpu_batch* b, bool reorder) {
     enqueue_lane(b, 1, b->side);  // Green's functions
     cudaEventRecord(b->ev_join, b->side);
     enqueue_lane(b, 2, s);       // deposit, assemble
-    if (reorder)
-        for (int m : b->members) ctx_enqueue_reorder(b->slots[m], s);
+    if (reorder) {  // beside the solve: the particles rest until the gather
+        cudaEventRecord(b->ev_dep, s);
+        cudaStreamWaitEvent(b->ref, b->ev_dep, 0);
+        for (int m : b->members) ctx_enqueue_reorder(b->slots[m], b->ref);
+        cudaEventRecord(b->ev_ref, b->ref);
+    }
     enqueue_lane(b, 6, s);       // FFT A, B
     cudaStreamWaitEvent(s, b->ev_join, 0);
     enqueue_lane(b, 3, s);       // FFT C, D, E, grad
@@ -390,6 +395,7 @@ int scgpu_batch_create(scgpu_batch** out, int device, int precision) {
         cudaStreamCreateWithPriority(&b->ref, cudaStreamNonBlocking, greatest) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_ref, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_dep, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&b->ev_t0) != cudaSuccess || cudaEventCreate(&b->ev_t1) != cudaSuccess) {
@@ -414,7 +420,7 @@ void scgpu_batch_destroy(scgpu_batch* b) {
     if (b->d_tab) cudaFree(b->d_tab);
     if (b->d_work) cudaFree(b->d_work);
     if (b->d_flags) cudaFree(b->d_flags);
-    for (cudaEvent_t e : {b->ev_fork, b->ev_join, b->ev_t0, b->ev_t1, b->ev_start, b->ev_ref})
+    for (cudaEvent_t e : {b->ev_fork, b->ev_join, b->ev_t0, b->ev_t1, b->ev_start, b->ev_ref, b->ev_dep})
         if (e) cudaEventDestroy(e);
     if (b->stream) cudaStreamDestroy(b->stream);
     if (b->xfer) cudaStreamDestroy(b->xfer);

@@ -1859,6 +1859,29 @@ __global__ void __launch_bounds__(kThreads) k_reorder(const uint32_t* __restrict
     }
 }
 
+// The permuted particles from the staging buffers back into the arrays (one
+// launch in place of seven copies), and the cell counts cleared for the next
+// sort.
+__global__ void __launch_bounds__(kThreads) k_reorder_back(double* __restrict__ x, double* __restrict__ y,
+                                                           double* __restrict__ z, double* __restrict__ px,
+                                                           double* __restrict__ py, double* __restrict__ pz,
+                                                           uint32_t* __restrict__ id, const double* __restrict__ sa,
+                                                           const double* __restrict__ sb,
+                                                           const uint32_t* __restrict__ sid, long long n,
+                                                           int* __restrict__ hist, int cells) {
+    const long long stride = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long p = first; p < n; p += stride) {
+        x[p] = sa[p];
+        y[p] = sa[n + p];
+        z[p] = sa[2 * n + p];
+        px[p] = sb[p];
+        py[p] = sb[n + p];
+        pz[p] = sb[2 * n + p];
+        id[p] = sid[p];
+    }
+    for (long long c = first; c < cells; c += stride) hist[c] = 0;
+}
+
 __global__ void __launch_bounds__(kThreads) k_iota(uint32_t* __restrict__ id, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         id[i] = (uint32_t)i;
@@ -2260,19 +2283,14 @@ void launch_soa_to_aos(const double* a, const double* b, const double* c, double
 }
 
 // Puts the particle arrays in cell order (the order of the last counting
-// sort); b.Ef / b.Bf / b.keys_alt are the staging buffers.
+// sort) and clears the cell counts; b.Ef / b.Bf / b.keys_alt are the staging
+// buffers.
 void launch_reorder(const DevBunch& b, cudaStream_t s) {
     const long long n = b.bc.N;
-    k_reorder<<<grid_for(n, 148 * 16), kThreads, 0, s>>>(b.vals, b.x, b.y, b.z, b.px, b.py, b.pz, b.id, b.Ef, b.Bf,
-                                                         b.keys_alt, n);
-    const size_t d = (size_t)n * sizeof(double);
-    cudaMemcpyAsync(b.x, b.Ef, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.y, b.Ef + n, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.z, b.Ef + 2 * n, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.px, b.Bf, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.py, b.Bf + n, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.pz, b.Bf + 2 * n, d, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(b.id, b.keys_alt, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+    const int g = grid_for(n, 148 * 16);
+    k_reorder<<<g, kThreads, 0, s>>>(b.vals, b.x, b.y, b.z, b.px, b.py, b.pz, b.id, b.Ef, b.Bf, b.keys_alt, n);
+    k_reorder_back<<<g, kThreads, 0, s>>>(b.x, b.y, b.z, b.px, b.py, b.pz, b.id, b.Ef, b.Bf, b.keys_alt, n, b.hist,
+                                          b.bc.n[0] * b.bc.n[1] * b.bc.n[2]);
 }
 
 void launch_iota(uint32_t* id, long long n, cudaStream_t s) { k_iota<<<grid_for(n, 148 * 16), kThreads, 0, s>>>(id, n); }

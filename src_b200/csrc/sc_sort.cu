@@ -4,7 +4,7 @@
 // sorts them:
 //   k_cell_keys (sc_particles.cu)  key and rank = atomicAdd(count[key], 1)
 //   exclusive scan of count         -> first sorted position of every cell
-//   k_scatter                       sorted key and particle index at start + rank
+//   k_scatter                       particle index at start + rank
 // The order of particles inside a cell depends on the order the atomics were
 // served in; the deposit therefore sums each cell exactly (fixed point), so
 // its result does not depend on that order and every run is bitwise the same.
@@ -70,13 +70,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const int* __restr
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ ranks,
-                                                 const int* __restrict__ start, uint32_t* __restrict__ skey,
-                                                 uint32_t* __restrict__ sval, long long n, int* __restrict__ err) {
+                                                 const int* __restrict__ start, uint32_t* __restrict__ sval, long long n,
+                                                 int* __restrict__ err) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const uint32_t k = keys[i];
         const long long p = (long long)start[k] + ranks[i];
         if (p >= 0 && p < n) {
-            skey[p] = k;
             sval[p] = (uint32_t)i;
         } else {
             atomicOr(err, kFlagSort);
@@ -101,14 +100,14 @@ void exclusive_scan(const int* in, int* out, long long n, int* blocks, cudaStrea
 }
 
 // After k_cell_keys: b.keys (key per particle), b.vals_alt (rank in its
-// cell), b.hist (count per cell).  Produces b.keys_alt (sorted keys) and
-// b.vals (particle index per sorted position); b.hist_scan holds the cell starts.
+// cell), b.hist (count per cell).  Produces b.vals (particle index per sorted
+// position); b.hist_scan holds the cell starts.
 void launch_sort(const DevBunch& b, cudaStream_t s) {
     const long long M = (long long)b.bc.n[0] * b.bc.n[1] * b.bc.n[2];
     exclusive_scan(b.hist, b.hist_scan, M, b.scan_blocks, s);
     long long g = (b.bc.N + 255) / 256;
     if (g > 148 * 16) g = 148 * 16;
-    k_scatter<<<(unsigned)g, 256, 0, s>>>(b.keys, b.vals_alt, b.hist_scan, b.keys_alt, b.vals, b.bc.N, &b.st->err);
+    k_scatter<<<(unsigned)g, 256, 0, s>>>(b.keys, b.vals_alt, b.hist_scan, b.vals, b.bc.N, &b.st->err);
 }
 
 }  // namespace sc
