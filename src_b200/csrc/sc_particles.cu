@@ -610,8 +610,14 @@ __device__ __forceinline__ void cic_charge(const double* d, double q, double* v)
 // Exact sums of the scattered charges (kFxFrac, fx_unit, node_density in
 // sc_exact.cuh).
 
-// A fixed-point charge t = rint(v) (|t| < 2^51; the conversion rounds half
-// to even, as rint) as two exact 32-bit limbs: hi = floor(t / 2^26) in
+// rint(v) for |v| < 2^51: adding 1.5 2^52 rounds half to even at the units bit
+// and leaves v in the mantissa's low bits (one addition on the FP64 pipe and
+// one on the integer units in place of a 64-bit conversion).
+__device__ __forceinline__ long long fx_round(double v) {
+    return __double_as_longlong(v + 0x1.8p52) - 0x4338000000000000ll;
+}
+
+// A fixed-point charge t = rint(v) (|t| < 2^51) as two exact 32-bit limbs: hi = floor(t / 2^26) in
 // [-2^25, 2^25) (arithmetic shift), lo = t - hi 2^26 in [0, 2^26).  Sums of
 // up to 32 limbs fit 32 bits (|sum hi| < 2^30, sum lo < 2^31) and recombine
 // exactly in 64 bits.
@@ -620,7 +626,7 @@ struct Limbs {
     unsigned lo;
 };
 __device__ __forceinline__ Limbs limbs_of(double v) {
-    const long long t = __double2ll_rn(v);
+    const long long t = fx_round(v);
     return Limbs{(int)(t >> 26), (unsigned)(t & 0x3ffffffll)};
 }
 __device__ __forceinline__ long long join(long long hi, long long lo) { return hi * (1ll << 26) + lo; }
@@ -666,12 +672,9 @@ __device__ __forceinline__ void deposit_body(const BunchConst& bc, const double*
                                              const int* __restrict__ bin, int nactive, StepState* st,
                                              unsigned long long* __restrict__ acc, VB g) {
     __shared__ MeshConsts ms;
-    __shared__ double qdt_s, to_int_s;
+    __shared__ double q_s;  // the charge in units of the fixed point: the unit is a power of two, no rounding
     load_mesh_consts(ms, st);
-    if (threadIdx.x == 0) {
-        qdt_s = st->qdt;
-        to_int_s = 1.0 / st->dep_unit;  // a power of two
-    }
+    if (threadIdx.x == 32) q_s = st->qdt / st->dep_unit;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int nx = bc.n[0], nxy = bc.n[0] * bc.n[1];
@@ -698,17 +701,16 @@ __device__ __forceinline__ void deposit_body(const BunchConst& bc, const double*
                 }
             }
             if (!cic_locate_r(m->hr, m->rhr, m->org, bc.n, X, l, d, PZ ? 1 : 0)) bad = true;
-            cic_charge(d, *fresh(&qdt_s), c);
+            cic_charge(d, *fresh(&q_s), c);
             key = (uint32_t)(l[0] + nx * l[1] + nxy * l[2]) + (uint32_t)bk * M;
             lz = l[2];
         } else {
 #pragma unroll
             for (int k = 0; k < 8; ++k) c[k] = 0.0;
         }
-        const double to_int = *fresh(&to_int_s);
         Limbs t[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] = limbs_of(c[k] * to_int);
+        for (int k = 0; k < 8; ++k) t[k] = limbs_of(c[k]);
         const unsigned group = __match_any_sync(kFull, key);
         const int gsize = __popc(group);
         const bool leader = lane == __ffs(group) - 1;
@@ -759,12 +761,9 @@ __device__ __forceinline__ void deposit_pairs_body(const BunchConst& bc, const d
                                                    const double* __restrict__ y, const double* __restrict__ z,
                                                    StepState* st, unsigned long long* __restrict__ acc, VB g) {
     __shared__ MeshConsts ms;
-    __shared__ double qdt_s, to_int_s;
+    __shared__ double q_s;  // the charge in units of the fixed point: the unit is a power of two, no rounding
     load_mesh_consts(ms, st);
-    if (threadIdx.x == 0) {
-        qdt_s = st->qdt;
-        to_int_s = 1.0 / st->dep_unit;  // a power of two
-    }
+    if (threadIdx.x == 32) q_s = st->qdt / st->dep_unit;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nx = bc.n[0], nxy = bc.n[0] * bc.n[1];
@@ -796,7 +795,7 @@ __device__ __forceinline__ void deposit_pairs_body(const BunchConst& bc, const d
             kb = (uint32_t)(lb[0] + nx * lb[1] + nxy * lb[2]);
         }
         const bool same = vb && ka == kb;
-        const double q = *fresh(&qdt_s), to_int = *fresh(&to_int_s);
+        const double q = *fresh(&q_s);
         long long T[8];
         {
             double c[8];
@@ -807,14 +806,14 @@ __device__ __forceinline__ void deposit_pairs_body(const BunchConst& bc, const d
                 for (int k = 0; k < 8; ++k) c[k] = 0.0;
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) T[k] = __double2ll_rn(c[k] * to_int);
+            for (int k = 0; k < 8; ++k) T[k] = fx_round(c[k]);
         }
         if (vb) {
             double c[8];
             cic_charge(db, q, c);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const long long t = __double2ll_rn(c[k] * to_int);
+                const long long t = fx_round(c[k]);
                 if (same) {
                     T[k] += t;
                 } else {
@@ -886,7 +885,6 @@ __global__ void __launch_bounds__(kThreads) k_deposit_bins(BunchConst bc, const 
 // in deposit_body.
 constexpr int kWeightFrac = 26;
 
-template <bool PZ>
 __device__ __forceinline__ void deposit_mixed_body(const BunchConst& bc, const double* __restrict__ x,
                                                    const double* __restrict__ y, double* __restrict__ z, StepState* st,
                                                    unsigned long long* __restrict__ acc, VB g) {
@@ -906,7 +904,7 @@ __device__ __forceinline__ void deposit_mixed_body(const BunchConst& bc, const d
         if (valid) {
             double X[3] = {x[i], y[i], z[i]};
             const MeshConsts* m = fresh(&ms);
-            if constexpr (PZ) {
+            {
                 const double w = wrap_z(X[2], m->org[2], m->org[2] + m->hr[2] * (double)bc.n[2]);
                 if (w != X[2]) {
                     z[i] = w;
@@ -915,7 +913,7 @@ __device__ __forceinline__ void deposit_mixed_body(const BunchConst& bc, const d
             }
             int l[3];
             float d[3];
-            if (!cic_locate_fast(m->rhr, m->org, bc.n, X, l, d, PZ ? 1 : 0)) bad = true;
+            if (!cic_locate_fast(m->rhr, m->org, bc.n, X, l, d, 1)) bad = true;
             const float u[3] = {1.0f - d[0], 1.0f - d[1], 1.0f - d[2]};
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -937,7 +935,7 @@ __device__ __forceinline__ void deposit_mixed_body(const BunchConst& bc, const d
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 const int node = (int)key + (k & 1) + ((k >> 1) & 1) * nx + ((k >> 2) & 1) * nxy;
-                if ((!PZ || (unsigned)(lz + (k >> 2)) < (unsigned)bc.n[2]) && t[k])
+                if ((unsigned)(lz + (k >> 2)) < (unsigned)bc.n[2] && t[k])
                     atomicAdd(acc + 2 * (long long)node, (unsigned long long)t[k]);
             }
         }
@@ -952,10 +950,97 @@ __device__ __forceinline__ void deposit_mixed_body(const BunchConst& bc, const d
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const int node = (int)key + (k & 1) + ((k >> 1) & 1) * nx + ((k >> 2) & 1) * nxy;
-                    if ((!PZ || (unsigned)(lz + (k >> 2)) < (unsigned)bc.n[2]) && sum[k])
+                    if ((unsigned)(lz + (k >> 2)) < (unsigned)bc.n[2] && sum[k])
                         atomicAdd(acc + 2 * (long long)node, (unsigned long long)sum[k]);
                 }
             }
+        }
+    }
+    if (bad) atomicOr(&st->err, kFlagGuard);
+}
+// Two particles per lane, as deposit_pairs_body: a pair in one cell enters the
+// warp's group reduction as the sum of its weights (at most 2^27 each, so 32
+// lanes' sums fit 32 bits unless every weight of a corner is exactly 1: such a
+// warp adds per lane).
+__device__ __forceinline__ void deposit_mixed_pairs_body(const BunchConst& bc, const double* __restrict__ x,
+                                                         const double* __restrict__ y, const double* __restrict__ z,
+                                                         StepState* st, unsigned long long* __restrict__ acc, VB g) {
+    __shared__ MeshConsts ms;
+    load_mesh_consts(ms, st);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nx = bc.n[0], nxy = bc.n[0] * bc.n[1];
+    const long long span = 2ll * blockDim.x;
+    bool bad = false;
+    auto weights = [&](const float* d, unsigned (&t)[8]) {
+        const float u[3] = {1.0f - d[0], 1.0f - d[1], 1.0f - d[2]};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float w = (k & 1 ? d[0] : u[0]) * (k & 2 ? d[1] : u[1]) * (k & 4 ? d[2] : u[2]);
+            t[k] = __float2uint_rn(w * 0x1p26f);
+        }
+    };
+    auto add = [&](uint32_t key, const unsigned (&t)[8]) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int node = (int)key + (k & 1) + ((k >> 1) & 1) * nx + ((k >> 2) & 1) * nxy;
+            if (t[k]) atomicAdd(acc + 2 * (long long)node, (unsigned long long)t[k]);
+        }
+    };
+    for (long long i0 = (long long)g.blk * span; i0 < bc.N; i0 += (long long)g.nblk * span) {
+        const long long ia = i0 + 64ll * warp + 2 * lane;
+        const bool va = ia < bc.N, vb = ia + 1 < bc.N;
+        double Xa[3] = {0.0, 0.0, 0.0}, Xb[3] = {0.0, 0.0, 0.0};
+        if (vb) {  // ia is even: the pair is one aligned 16-byte load per coordinate
+            const double2 px = *reinterpret_cast<const double2*>(x + ia);
+            const double2 py = *reinterpret_cast<const double2*>(y + ia);
+            const double2 pz = *reinterpret_cast<const double2*>(z + ia);
+            Xa[0] = px.x, Xa[1] = py.x, Xa[2] = pz.x;
+            Xb[0] = px.y, Xb[1] = py.y, Xb[2] = pz.y;
+        } else if (va) {
+            Xa[0] = x[ia], Xa[1] = y[ia], Xa[2] = z[ia];
+        }
+        uint32_t key = 0xffffffffu;
+        unsigned T[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        const MeshConsts* m = fresh(&ms);
+        if (va) {
+            int l[3];
+            float d[3];
+            if (!cic_locate_fast(m->rhr, m->org, bc.n, Xa, l, d, 0)) bad = true;
+            key = (uint32_t)(l[0] + nx * l[1] + nxy * l[2]);
+            weights(d, T);
+        }
+        if (vb) {
+            int l[3];
+            float d[3];
+            if (!cic_locate_fast(m->rhr, m->org, bc.n, Xb, l, d, 0)) bad = true;
+            const uint32_t kb = (uint32_t)(l[0] + nx * l[1] + nxy * l[2]);
+            unsigned t[8];
+            weights(d, t);
+            if (kb == key) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) T[k] += t[k];
+            } else {
+                add(kb, t);
+            }
+        }
+        unsigned most = T[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) most = max(most, T[k]);
+        const unsigned group = __match_any_sync(kFull, key);
+        const int gsize = __popc(group);
+        const bool leader = lane == __ffs(group) - 1;
+        unsigned multi = __ballot_sync(kFull, leader && gsize > 1);
+        const bool passes = __popc(multi) <= kMaxGroupPasses && !__any_sync(kFull, most >= 1u << 27);
+        if (va && (gsize == 1 || !passes)) add(key, T);
+        while (passes && multi) {
+            const int ld = __ffs(multi) - 1;
+            multi &= multi - 1;
+            const bool in = (__shfl_sync(kFull, group, ld) >> lane) & 1u;
+            unsigned sum[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sum[k] = __reduce_add_sync(kFull, in ? T[k] : 0u);
+            if (va && lane == ld) add(key, sum);
         }
     }
     if (bad) atomicOr(&st->err, kFlagGuard);
@@ -964,7 +1049,10 @@ template <bool PZ>
 __global__ void __launch_bounds__(kThreads) k_deposit_mixed(BunchConst bc, const double* __restrict__ x,
                                                             const double* __restrict__ y, double* __restrict__ z,
                                                             StepState* st, unsigned long long* __restrict__ acc) {
-    deposit_mixed_body<PZ>(bc, x, y, z, st, acc, vb_grid());
+    if constexpr (PZ)
+        deposit_mixed_body(bc, x, y, z, st, acc, vb_grid());
+    else
+        deposit_mixed_pairs_body(bc, x, y, z, st, acc, vb_grid());
 }
 
 // rho = (exact node sum) / dT * tmp2   (PartBunch.cpp:496, :510-511); the
@@ -1939,7 +2027,7 @@ __global__ void __launch_bounds__(NT) k_deposit_batch(const DevBunch* __restrict
     const int4 w = resolve_block(work, nitems);
     const DevBunch& d = tab[w.x];
     if constexpr (MIXED)
-        deposit_mixed_body<false>(d.bc, d.x, d.y, d.z, d.st, d.nacc, VB{w.y, w.w});
+        deposit_mixed_pairs_body(d.bc, d.x, d.y, d.z, d.st, d.nacc, VB{w.y, w.w});
     else
         deposit_pairs_body(d.bc, d.x, d.y, d.z, d.st, d.nacc, VB{w.y, w.w});
 }
