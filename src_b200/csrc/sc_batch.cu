@@ -186,7 +186,17 @@ int rebuild(scgpu_batch* b) {
     };
     auto cells = [](const DevBunch& d) { return (long long)d.bc.n[0] * d.bc.n[1] * d.bc.n[2]; };
     const int dep = b->dep_threads;
-    add_per_bunch(0, kBatchDrift, [](const DevBunch& d) { return d.red_blocks; });
+    // Particle kernels: as many particles per thread, in every bunch, as fill
+    // the resident blocks once (148 SMs, three blocks of 256), so a block's
+    // set-up and reduction serve several passes; at most 16, so that large
+    // bunches still spread over enough blocks to balance small ones.
+    long long particle_blocks = 0;
+    for (const DevBunch& d : tab) particle_blocks += (d.bc.N + 255) / 256;
+    const long long per_thread = std::min<long long>(16, std::max<long long>(1, particle_blocks / (148 * 3)));
+    auto particle_grid = [per_thread](const DevBunch& d) {
+        return (int)std::min<long long>((d.bc.N + 256 * per_thread - 1) / (256 * per_thread), d.red_blocks);
+    };
+    add_per_bunch(0, kBatchDrift, particle_grid);
     add_per_bunch(1, kBatchIgfTmp, [](const DevBunch& d) {
         return blocks_for((long long)(d.bc.n[0] + 2) * (d.bc.n[1] + 2) * (d.bc.n[2] + 2), 256, kCellGridCap);
     });
@@ -195,7 +205,8 @@ int rebuild(scgpu_batch* b) {
     add_pass(1, kPassDctY);
     add_pass(1, kPassDctX);
     add_pass(1, kPassDctPlane);
-    add_per_bunch(2, kBatchDeposit, [dep](const DevBunch& d) { return blocks_for(d.bc.N, dep, 148 * 8 * 256 / dep); });
+    // (the deposit keeps one block per 512 particles: two per lane, no reduction)
+    add_per_bunch(2, kBatchDeposit, [dep](const DevBunch& d) { return blocks_for((d.bc.N + 1) / 2, dep, 148 * 8 * 256 / dep); });
     add_per_bunch(2, kBatchAssemble, [&](const DevBunch& d) { return blocks_for(cells(d), 256, kCellGridCap); });
     add_per_bunch(4, kBatchAdvance, [](const DevBunch&) { return 1; });
     add_pass(6, kPassZR2C);
@@ -208,7 +219,7 @@ int rebuild(scgpu_batch* b) {
     add_per_bunch(3, kBatchGrad, [](const DevBunch& d) {
         return (int)std::min<long long>(((long long)d.bc.n[0] * d.bc.n[1] + 255) / 256 * d.bc.n[2], kCellGridCap);
     });
-    add_per_bunch(5, kBatchGather, [](const DevBunch& d) { return d.red_blocks; });
+    add_per_bunch(5, kBatchGather, particle_grid);
     if (nm > b->tab_cap) {
         if (b->d_tab) cudaFree(b->d_tab);
         if (b->d_flags) cudaFree(b->d_flags);

@@ -2069,9 +2069,11 @@ __global__ void __launch_bounds__(kThreads) k_grad_batch(const DevBunch* __restr
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 3) k_gather_batch(const DevBunch* __restrict__ tab, const int4* __restrict__ work, int nitems) {
+    extern __shared__ __align__(16) double gather_sm[];
     const int4 w = resolve_block(work, nitems);
     const DevBunch& d = tab[w.x];
-    gather_body<T>(d.bc, d.x, d.y, d.z, d.px, d.py, d.pz, (const T*)d.E4, d.st, d.partials, d.ticket, VB{w.y, w.w});
+    gather_body<T, false, false, true>(d.bc, d.x, d.y, d.z, d.px, d.py, d.pz, (const T*)d.E4, d.st, d.partials, d.ticket,
+                                       VB{w.y, w.w}, nullptr, gather_sm);
 }
 
 }  // namespace
@@ -2114,9 +2116,9 @@ void launch_batch(int kind, int precision, int threads, const DevBunch* tab, con
             break;
         case kBatchGather:
             if (f64)
-                k_gather_batch<double><<<nblocks, kThreads, 0, s>>>(tab, work, nitems);
+                k_gather_batch<double><<<nblocks, kThreads, kGatherSmem, s>>>(tab, work, nitems);
             else
-                k_gather_batch<float><<<nblocks, kThreads, 0, s>>>(tab, work, nitems);
+                k_gather_batch<float><<<nblocks, kThreads, kGatherSmem, s>>>(tab, work, nitems);
             break;
         default: break;
     }
