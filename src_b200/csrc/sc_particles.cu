@@ -376,44 +376,25 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
     __syncthreads();
     const bool push = DRIFT && pushed_s == 0;  // else the gather of the step before has pushed R
     double v[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};  // min x,y,z, -max x,y,z
-    // The next particle's loads are issued before the current one is
-    // computed, so each thread keeps two particles' reads in flight.
     const long long stride = (long long)g.nblk * blockDim.x;
     long long i = g.blk * (long long)blockDim.x + threadIdx.x;
-    double Rn[3] = {0.0, 0.0, 0.0}, Pn[3] = {0.0, 0.0, 0.0};
-    if (i < bc.N) {
-        Rn[0] = x[i], Rn[1] = y[i], Rn[2] = z[i];
-        if (push) Pn[0] = px[i], Pn[1] = py[i], Pn[2] = pz[i];
-    }
-    for (; i < bc.N; i += stride) {
-        double R[3] = {Rn[0], Rn[1], Rn[2]};
-        const double P[3] = {Pn[0], Pn[1], Pn[2]};
-        const long long j = i + stride;
-        if (j < bc.N) {
-            Rn[0] = x[j], Rn[1] = y[j], Rn[2] = z[j];
-            if (push) Pn[0] = px[j], Pn[1] = py[j], Pn[2] = pz[j];
-        }
+    // frame change, store and bounds of one particle
+    auto finish = [&](long long k, double* R) {
         if constexpr (DRIFT) {
             double b[3];
+            const Trafo* t = fresh(&r2b_s);
             if constexpr (MIXED) {
-                if (push) mixed_push(R, mixed_push_factor(P, bc.s_cdt), P);
-                const Trafo* t = fresh(&r2b_s);
                 const double X[3] = {R[0] - t->origin[0], R[1] - t->origin[1], R[2] - t->origin[2]};
                 matvec_fma(t->M, X, b);
             } else {
-                if (push) {
-                    double step[3];
-                    push_step(P, step);
-                    push_move(R, step, bc.s_cdt, bc.rs_cdt);
-                }
-                trafo_transform_to(*fresh(&r2b_s), R, b);
+                trafo_transform_to(*t, R, b);
             }
             R[0] = b[0];
             R[1] = b[1];
             R[2] = b[2];
-            x[i] = R[0];
-            y[i] = R[1];
-            z[i] = R[2];
+            x[k] = R[0];
+            y[k] = R[1];
+            z[k] = R[2];
         }
         v[0] = fmin(v[0], R[0]);
         v[1] = fmin(v[1], R[1]);
@@ -421,6 +402,31 @@ __device__ __forceinline__ void drift_body(const BunchConst& bc, double* __restr
         v[3] = fmin(v[3], -R[0]);
         v[4] = fmin(v[4], -R[1]);
         v[5] = fmin(v[5], -R[2]);
+    };
+    // The next particle's loads are issued before the current one is
+    // computed, so each thread keeps two particles' reads in flight.
+    if (!push) {
+        double Rn[3] = {0.0, 0.0, 0.0};
+        if (i < bc.N) Rn[0] = x[i], Rn[1] = y[i], Rn[2] = z[i];
+        for (; i < bc.N; i += stride) {
+            double R[3] = {Rn[0], Rn[1], Rn[2]};
+            const long long j = i + stride;
+            if (j < bc.N) Rn[0] = x[j], Rn[1] = y[j], Rn[2] = z[j];
+            finish(i, R);
+        }
+    } else {
+        for (; i < bc.N; i += stride) {
+            double R[3] = {x[i], y[i], z[i]};
+            const double P[3] = {px[i], py[i], pz[i]};
+            if constexpr (MIXED) {
+                mixed_push(R, mixed_push_factor(P, bc.s_cdt), P);
+            } else {
+                double step[3];
+                push_step(P, step);
+                push_move(R, step, bc.s_cdt, bc.rs_cdt);
+            }
+            finish(i, R);
+        }
     }
     bounds_tail(bc, v, st, mesh_in_s, partials, ticket, g);
 }
@@ -462,7 +468,7 @@ __device__ __forceinline__ void bounds_tail(const BunchConst& bc, double (&v)[6]
     }
 }
 template <bool DRIFT, bool MIXED = false>
-__global__ void __launch_bounds__(kThreads, 3) k_drift_to_beam(BunchConst bc, double* __restrict__ x, double* __restrict__ y,
+__global__ void __launch_bounds__(kThreads, 4) k_drift_to_beam(BunchConst bc, double* __restrict__ x, double* __restrict__ y,
                                                             double* __restrict__ z, const double* __restrict__ px,
                                                             const double* __restrict__ py, const double* __restrict__ pz,
                                                             StepState* st, double* partials, unsigned* ticket) {
