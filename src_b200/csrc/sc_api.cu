@@ -30,7 +30,7 @@ static GetAddressRangeFn address_range_fn() {
     return fn;
 }
 
-bool device_buffer_ok(const void* p, size_t bytes, int device, std::string* why) {
+bool device_buffer_ok(const void* p, size_t bytes, int device, std::string* why, bool* managed) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
@@ -46,6 +46,7 @@ bool device_buffer_ok(const void* p, size_t bytes, int device, std::string* why)
         *why = "host memory, not device memory";
         return false;
     }
+    if (managed) *managed = a.type == cudaMemoryTypeManaged;
     if (GetAddressRangeFn fn = address_range_fn()) {
         unsigned long long base = 0;
         size_t size = 0;
@@ -731,85 +732,71 @@ int scgpu_unregister_host(scgpu_ctx* c, void* ptr) {
     return SCGPU_OK;
 }
 
-static int compute_potential_impl(scgpu_ctx* c, double* rho, const double hr[3], bool device_ptr) {
-    if (!c || !rho || !hr) return fail(c, SCGPU_ERR_ARG, "null argument");
-    for (int d = 0; d < 3; ++d)
-        if (!(hr[d] > 0.0) || !std::isfinite(hr[d])) return fail(c, SCGPU_ERR_ARG, "hr must be positive and finite");
-    CK(cudaSetDevice(c->device));
-    DevBunch& b = c->b;
-    cudaStream_t s = c->stream;
-    const long long M = (long long)b.bc.n[0] * b.bc.n[1] * b.bc.n[2];
-    if (device_ptr) {
-        std::string why;
-        if (!device_buffer_ok(rho, (size_t)M * sizeof(double), c->device, &why))
-            return fail(c, SCGPU_ERR_ARG, "rho_inout_device: " + why);
-    }
-    const cudaMemcpyKind in_kind = device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    const cudaMemcpyKind out_kind = device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpyAsync(b.st->hr_scaled, hr, 3 * sizeof(double), cudaMemcpyHostToDevice, s));
-    if (b.precision == SCGPU_PLAIN_FP64) {
-        CK(cudaMemcpyAsync(b.rho, rho, M * sizeof(double), in_kind, s));
+// The Green's function beside what only needs rho (on `main`, until the
+// convolution needs its spectrum): on the side stream from here, as in a step.
+static void fork_green(scgpu_ctx* c, bool image, cudaStream_t main) {
+    cudaEventRecord(c->ev_fork, main);
+    cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+    if (image) {
+        launch_igf_image(c->b, c->side);
+        launch_green_transform_image(c->b, c->side);
     } else {
-        double* stage = c->capacity * 3 >= M ? b.Ef : nullptr;
-        bool tmp_alloc = false;
-        if (!stage) {
-            CK(cudaMalloc(&stage, M * sizeof(double)));
-            tmp_alloc = true;
-        }
-        CK(cudaMemcpyAsync(stage, rho, M * sizeof(double), in_kind, s));
-        launch_f64_to_f32(stage, (float*)b.rho, M, s);
-        if (tmp_alloc) {
-            CK(cudaStreamSynchronize(s));
-            cudaFree(stage);
-        }
+        enqueue_green(c, c->side);
     }
-    enqueue_green(c, s);
-    launch_convolution(b, kConvPotential, s);
-    CK(cudaMemcpyAsync(rho, b.phi, M * sizeof(double), out_kind, s));
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(s));
-    c->have_solve = false;
-    return SCGPU_OK;
+    cudaEventRecord(c->ev_join, c->side);
 }
 
-// computePotential(rho, hr, zshift) (FFTPoissonSolver.cpp:287-327): the
-// image charge's potential, through the shifted Green's function.
-static int compute_potential_image_impl(scgpu_ctx* c, double* rho, const double hr[3], double zshift, bool device_ptr) {
+// computePotential(rho, hr) (FFTPoissonSolver.cpp:337-382), or with `image`
+// computePotential(rho, hr, zshift) (:287-327): the image charge's potential,
+// through the shifted Green's function.  The Green's function is the longer
+// half, so the copy in and passes A, B run beside it, and a device buffer is
+// transformed from and back into in place, which saves two copies (the mixed
+// form converts it first): a solve on the device takes 51 us at 16^3 (60 one
+// after the other, with the copies), 88 at 40 x 20 x 60 (107), 303 at 128^3
+// (330).  A host buffer, managed memory (its pages would move one by one) and
+// a buffer not aligned to its elements go through the context's grids.
+static int solve_impl(scgpu_ctx* c, double* rho, const double hr[3], bool image, double zshift, bool device_ptr) {
     if (!c || !rho || !hr) return fail(c, SCGPU_ERR_ARG, "null argument");
     for (int d = 0; d < 3; ++d)
         if (!(hr[d] > 0.0) || !std::isfinite(hr[d])) return fail(c, SCGPU_ERR_ARG, "hr must be positive and finite");
-    if (!std::isfinite(zshift)) return fail(c, SCGPU_ERR_ARG, "zshift must be finite");
-    if (c->b.periodic_z) return fail(c, SCGPU_ERR_UNSUPPORTED, "image charges with periodic z");
-    CK(cudaSetDevice(c->device));
-    if (device_ptr) {
-        std::string why;
-        if (!device_buffer_ok(rho, (size_t)mesh_cells(c->b) * sizeof(double), c->device, &why))
-            return fail(c, SCGPU_ERR_ARG, "rho_inout_device: " + why);
+    if (image) {
+        if (!std::isfinite(zshift)) return fail(c, SCGPU_ERR_ARG, "zshift must be finite");
+        if (c->b.periodic_z) return fail(c, SCGPU_ERR_UNSUPPORTED, "image charges with periodic z");
     }
-    int rc = ensure_image(c);
-    if (rc) return rc;
+    CK(cudaSetDevice(c->device));
     DevBunch& b = c->b;
     cudaStream_t s = c->stream;
     const long long M = mesh_cells(b);
+    bool managed = false;
+    if (device_ptr) {
+        std::string why;
+        if (!device_buffer_ok(rho, (size_t)M * sizeof(double), c->device, &why, &managed))
+            return fail(c, SCGPU_ERR_ARG, "rho_inout_device: " + why);
+    }
+    if (image) {
+        int rc = ensure_image(c);
+        if (rc) return rc;
+    }
+    const bool in_place = device_ptr && !managed && reinterpret_cast<uintptr_t>(rho) % sizeof(double) == 0;
     const cudaMemcpyKind in_kind = device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const cudaMemcpyKind out_kind = device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpyAsync(b.st->hr_scaled, hr, 3 * sizeof(double), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(&b.st->zshift, &zshift, sizeof(double), cudaMemcpyHostToDevice, s));
+    launch_set_solve(b, hr, zshift, s);
+    fork_green(c, image, s);
+    DevBunch v = b;  // the solve's view: rho in, the potential out
+    if (in_place) v.phi = rho;
     if (b.precision == SCGPU_PLAIN_FP64) {
-        CK(cudaMemcpyAsync(b.rho, rho, M * sizeof(double), in_kind, s));
-    } else {
-        double* stage = nullptr;
-        CK(cudaMalloc(&stage, M * sizeof(double)));
-        cudaError_t e = cudaMemcpyAsync(stage, rho, M * sizeof(double), in_kind, s);
-        if (e == cudaSuccess) launch_f64_to_f32(stage, (float*)b.rho, M, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        cudaFree(stage);
-        if (e != cudaSuccess) return cuda_fail(c, e, "staging rho");
+        if (in_place)
+            v.rho = rho;
+        else
+            CK(cudaMemcpyAsync(b.rho, rho, M * sizeof(double), in_kind, s));
+    } else {  // without a buffer to convert from, the potential's grid is free until the last pass
+        if (!in_place) CK(cudaMemcpyAsync(b.phi, rho, M * sizeof(double), in_kind, s));
+        launch_f64_to_f32(v.phi, (float*)b.rho, M, s);
     }
-    launch_igf_image(b, s);
-    launch_green_transform_image(b, s);
-    launch_convolution_part(b, kConvPotential, kConvForwardPart | kConvImagePart, s);
-    CK(cudaMemcpyAsync(rho, b.phi, M * sizeof(double), out_kind, s));
+    launch_convolution_part(v, kConvPotential, kConvForwardPart, s);
+    CK(cudaStreamWaitEvent(s, c->ev_join, 0));
+    launch_convolution_part(v, kConvPotential, image ? kConvImagePart : kConvRestPart, s);
+    if (!in_place) CK(cudaMemcpyAsync(rho, b.phi, M * sizeof(double), out_kind, s));
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
     c->have_solve = false;
@@ -1127,17 +1114,19 @@ int scgpu_set_periodic_z(scgpu_ctx* c, int periodic) {
 }
 
 int scgpu_compute_potential_image(scgpu_ctx* c, double* rho, const double hr[3], double zshift) {
-    return compute_potential_image_impl(c, rho, hr, zshift, false);
+    return solve_impl(c, rho, hr, true, zshift, false);
 }
 
 int scgpu_compute_potential_image_device(scgpu_ctx* c, double* rho, const double hr[3], double zshift) {
-    return compute_potential_image_impl(c, rho, hr, zshift, true);
+    return solve_impl(c, rho, hr, true, zshift, true);
 }
 
-int scgpu_compute_potential(scgpu_ctx* c, double* rho, const double hr[3]) { return compute_potential_impl(c, rho, hr, false); }
+int scgpu_compute_potential(scgpu_ctx* c, double* rho, const double hr[3]) {
+    return solve_impl(c, rho, hr, false, 0.0, false);
+}
 
 int scgpu_compute_potential_device(scgpu_ctx* c, double* rho, const double hr[3]) {
-    return compute_potential_impl(c, rho, hr, true);
+    return solve_impl(c, rho, hr, false, 0.0, true);
 }
 
 int scgpu_compute_self_fields(scgpu_ctx* c, long long n, const double* R, const double* P, double* q_macro, double dT,
@@ -1166,13 +1155,14 @@ int scgpu_compute_self_fields(scgpu_ctx* c, long long n, const double* R, const 
     STAGE("reduce_state");
     launch_drift_to_beam(b, false, s);
     STAGE("bounds");
-    enqueue_green(c, s);
-    STAGE("green");
+    fork_green(c, false, s);
     launch_deposit(b, s);
     STAGE("deposit");
     launch_assemble_rho(b, s);
+    launch_convolution_part(b, kConvSelfField, kConvForwardPart, s);
     STAGE("assemble");
-    launch_convolution(b, kConvSelfField, s);
+    CK(cudaStreamWaitEvent(s, c->ev_join, 0));
+    launch_convolution_part(b, kConvSelfField, kConvRestPart, s);
     STAGE("convolution");
     launch_grad(b, s);
     STAGE("grad");

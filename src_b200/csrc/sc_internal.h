@@ -86,7 +86,7 @@ FftPlan make_plan(int L);
 // before anything is enqueued, so a host or foreign pointer becomes
 // SCGPU_ERR_ARG instead of an illegal-address fault on the GPU.  *why says
 // what is wrong.
-bool device_buffer_ok(const void* p, size_t bytes, int device, std::string* why);
+bool device_buffer_ok(const void* p, size_t bytes, int device, std::string* why, bool* managed = nullptr);
 // a 2D (r, z) field map (sc_fieldmap.cpp): grid points, ranges [m], the
 // frequency [MHz] of a dynamic map, and the values (Bz, Br or Ez, Er, Bt)
 int fieldmap_2d(const char* path, bool* dynamic, int* nz, int* nr, double* zbegin, double* zend, double* rbegin,
@@ -107,6 +107,7 @@ void prime_particle_grids();  // occupancy of the particle kernels, before any c
 void launch_reduce_state(const DevBunch& b, bool init_frame, cudaStream_t s);
 // mixed: the mixed form's half drift and frame change (fused multiply-adds)
 void launch_drift_to_beam(const DevBunch& b, bool drift, cudaStream_t s, bool mixed = false);
+void launch_set_solve(const DevBunch& b, const double hr[3], double zshift, cudaStream_t s);
 void launch_advance_reference(const DevBunch& b, cudaStream_t s);
 void launch_cell_keys(const DevBunch& b, int digit_bits, cudaStream_t s);
 void launch_deposit(const DevBunch& b, cudaStream_t s);

@@ -1177,6 +1177,14 @@ __global__ void k_finish_psum(BunchConst bc, StepState* st, int frame, int advan
     if (advance) s.step += 1;
 }
 
+// hr_scaled and zshift of a stand-alone solve (kernel arguments: no staged copy)
+__global__ void k_set_solve(StepState* st, double h0, double h1, double h2, double zshift) {
+    st->hr_scaled[0] = h0;
+    st->hr_scaled[1] = h1;
+    st->hr_scaled[2] = h2;
+    st->zshift = zshift;
+}
+
 __global__ void k_finish_stats(StepState* st) {
     if (blockIdx.x != 0 || threadIdx.x >= 28) return;
     const double v = ex_to_double(get_limbs(st->xlimbs + 4 * threadIdx.x));
@@ -2325,6 +2333,10 @@ void launch_gather_fields(const DevBunch& b, cudaStream_t s) {
         k_gather_fields<double><<<b.red_blocks, kThreads, 0, s>>>(b.bc, b.x, b.y, b.z, (const double*)b.E4, b.st, b.Ef, b.Bf);
     else
         k_gather_fields<float><<<b.red_blocks, kThreads, 0, s>>>(b.bc, b.x, b.y, b.z, (const float*)b.E4, b.st, b.Ef, b.Bf);
+}
+
+void launch_set_solve(const DevBunch& b, const double hr[3], double zshift, cudaStream_t s) {
+    k_set_solve<<<1, 1, 0, s>>>(b.st, hr[0], hr[1], hr[2], zshift);
 }
 
 void launch_finish_mesh(const DevBunch& b, cudaStream_t s) { k_finish_mesh<<<1, 32, 0, s>>>(b.bc, b.st); }

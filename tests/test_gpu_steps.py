@@ -142,3 +142,33 @@ def test_batch_of_many_bunches_equals_single_steps(gpu):
             got.append([a for s in slots for a in b.member(s).download()])
     for a, c in zip(*got):
         np.testing.assert_array_equal(a, c)
+
+
+@pytest.mark.parametrize("nr", [(16, 16, 16), (20, 12, 9)])
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+@pytest.mark.parametrize("image", [False, True])
+def test_device_solve_in_place(gpu, nr, form, image):
+    """A device buffer solved in place, and one that is not aligned to its
+    elements (through the context's grids), give the host call's bits."""
+    import ctypes as C
+
+    import torch
+
+    prec = gpu.MIXED if form == "mixed" else gpu.PLAIN_FP64
+    rho = np.random.default_rng(11).standard_normal(nr[::-1])
+    hr = (C.c_double * 3)(1e-3, 1.5e-3, 0.7e-3)
+    zs = -3e-3
+    L = gpu.lib()
+    with gpu.Context(nr, precision=prec) as c:
+        want = c.compute_potential_image(rho, hr, zs) if image else c.compute_potential(rho, hr)
+        raw = torch.empty(8 * rho.size + 16, dtype=torch.uint8, device="cuda")
+        for shift in (0, 8, 4):
+            buf = raw[shift:shift + 8 * rho.size]
+            buf.copy_(torch.from_numpy(rho.reshape(-1).view(np.uint8)))
+            torch.cuda.synchronize()
+            p = C.c_void_p(buf.data_ptr())
+            rc = (L.scgpu_compute_potential_image_device(c.h, p, hr, zs) if image
+                  else L.scgpu_compute_potential_device(c.h, p, hr))
+            assert rc == 0
+            got = buf.cpu().numpy().view(np.float64).reshape(rho.shape)
+            np.testing.assert_array_equal(got, want)
