@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_fft_x_conv(const Cx<TI>* in, 
     fft_x_conv_body<TI, TO, LT, NC, NT, CG>(in, out, ghat, n0, n1, L1, rows, px, twi, two, blockIdx.x);
 }
 
-// Pass C on rows of L = 2 n0 points: 8 threads per row.  The forward
-// transform leaves each thread the spectrum at a + 8m, exactly the inputs
+// Pass C on rows of L = 2 n0 points: TL threads per row.  The forward
+// transform leaves each thread the spectrum at a + TL m, exactly the inputs
 // the inverse transform's first stages need from it.
 template <typename TI, typename TO, bool CG, int L>
 __device__ __forceinline__ void fft_x_conv_lines_body(const Cx<TI>* in, Cx<TO>* out, const TI* __restrict__ ghat, int n0,
@@ -444,13 +444,13 @@ __device__ __forceinline__ void fft_x_conv_lines_body(const Cx<TI>* in, Cx<TO>* 
     using G = LineGeo<L>;
     constexpr int M = G::M;
     __shared__ __align__(16) CO xbuf[G::LINES][G::BUF];
-    const int li = threadIdx.x >> 3, a = threadIdx.x & 7;
+    const int li = threadIdx.x / G::TL, a = threadIdx.x % G::TL;
     const int r = blk * G::LINES + li;
     const bool live = r < rows;
     CI v[M];
 #pragma unroll
     for (int m = 0; m < M; ++m)
-        v[m] = (live && m < M / 2) ? in[(size_t)r * L + a + 8 * m] : CI{(TI)0, (TI)0};
+        v[m] = (live && m < M / 2) ? in[(size_t)r * L + a + G::TL * m] : CI{(TI)0, (TI)0};
     const int kz = live ? r / L1 : 0;
     const int ky = live ? r - kz * L1 : 0;
     const int gy = ky <= n1 ? ky : L1 - ky;
@@ -461,7 +461,7 @@ __device__ __forceinline__ void fft_x_conv_lines_body(const Cx<TI>* in, Cx<TO>* 
     GV g[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        const int kx = a + 8 * m;
+        const int kx = a + G::TL * m;
         const int gx = kx <= n0 ? kx : L - kx;
         g[m] = live ? reinterpret_cast<const GV*>(ghat)[grow + gx] : GV{};
     }
@@ -481,7 +481,7 @@ __device__ __forceinline__ void fft_x_conv_lines_body(const Cx<TI>* in, Cx<TO>* 
     line_fft<TO, true, false, L>(w, a, xbuf[li], two);
     if (!live) return;
 #pragma unroll
-    for (int m = 0; m < M / 2; ++m) out[(size_t)r * L + a + 8 * m] = w[m];  // x < n0
+    for (int m = 0; m < M / 2; ++m) out[(size_t)r * L + a + G::TL * m] = w[m];  // x < n0
 }
 
 template <typename TI, typename TO, bool CG, int L>
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_x_conv_lines(const Cx<TI
 }
 
 // Passes B (forward, inputs y < L/2) and D (inverse, outputs y < L/2) on
-// columns of L points along y: 8 threads per column (in different warps),
+// columns of L points along y: TL threads per column (in different warps),
 // consecutive x of one plane per block.
 template <typename T, bool INV, int L>
 __device__ __forceinline__ void fft_y_lines_body(Cx<T>* __restrict__ spec, int n0, int L0, int planes,
@@ -512,12 +512,12 @@ __device__ __forceinline__ void fft_y_lines_body(Cx<T>* __restrict__ spec, int n
     C v[M];
 #pragma unroll
     for (int m = 0; m < M; ++m)
-        v[m] = (live && (INV || m < M / 2)) ? col[(size_t)(a + 8 * m) * L0] : C{(T)0, (T)0};
+        v[m] = (live && (INV || m < M / 2)) ? col[(size_t)(a + G::TL * m) * L0] : C{(T)0, (T)0};
     line_fft<T, INV, !INV, L, true>(v, a, xbuf[li], twy);
     if (!live) return;
     constexpr int MO = INV ? M / 2 : M;  // D keeps y < L/2
 #pragma unroll
-    for (int m = 0; m < MO; ++m) col[(size_t)(a + 8 * m) * L0] = v[m];
+    for (int m = 0; m < MO; ++m) col[(size_t)(a + G::TL * m) * L0] = v[m];
 }
 
 template <typename T, bool INV, int L>
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_y_lines(Cx<T>* __restric
 }
 
 // Pass A on z lines of L = 2 n2 points: two real columns (x, x + 1) of one y
-// per complex line, 8 threads per line with the lanes along x (consecutive
+// per complex line, TL threads per line with the lanes along x (consecutive
 // column pairs, so a warp reads and writes whole rows) and block-level
 // exchanges.  The two half spectra need Z[k] and Z[L - k], which sit in
 // different threads: the transformed line goes through its buffer once more.
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_z_r2c_lines(const T* __r
     for (int m = 0; m < M; ++m) {
         v[m] = C{(T)0, (T)0};
         if (live && m < M / 2) {
-            const T* p = rho + ((size_t)(a + 8 * m) * n1 + y) * n0 + x;
+            const T* p = rho + ((size_t)(a + G::TL * m) * n1 + y) * n0 + x;
             v[m].x = p[0];
             if (odd) v[m].y = p[1];
         }
@@ -558,12 +558,12 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_z_r2c_lines(const T* __r
     C* xs = xbuf[li];
     line_fft<T, false, true, L, true>(v, a, xs, twz);
 #pragma unroll
-    for (int m = 0; m < M; ++m) xs[xidx<L>(a + 8 * m)] = v[m];
+    for (int m = 0; m < M; ++m) xs[xidx<L>(a + G::TL * m)] = v[m];
     __syncthreads();
     if (!live) return;
 #pragma unroll
     for (int m = 0; m <= M / 2; ++m) {
-        const int k = a + 8 * m;
+        const int k = a + G::TL * m;
         if (k > K) break;
         const C Z = xs[xidx<L>(k)];
         const C Zm = xs[xidx<L>(k == 0 ? 0 : L - k)];
@@ -712,17 +712,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dct_lines(const double* __res
 
 // The same cosine transforms for 256-point extensions with the
 // register-resident line transform: two real lines per complex line (lines
-// 2p and 2p + 1 as its real and imaginary parts, as in dct_lines_body), 8
+// 2p and 2p + 1 as its real and imaginary parts, as in dct_lines_body), 16
 // threads per complex line with the lanes along p, so one access reads
-// consecutive lines; thread a holds the extension's elements a + 8m.  The
+// consecutive lines; thread a holds the extension's elements a + TL m.  The
 // butterflies, twiddles and operation order are block_fft's, so Ĝ has the
 // same bits.
 template <typename TO, int L>
-__global__ void __launch_bounds__(LineGeo<L>::NT) k_dct_lines_reg(const double* __restrict__ in, TO* __restrict__ out,
+__global__ void __launch_bounds__(LineGeo<L, 16>::NT, 4) k_dct_lines_reg(const double* __restrict__ in, TO* __restrict__ out,
                                                                  int len, int nb, long long sb, long long so,
                                                                  long long se, const double2* __restrict__ twd) {
     using C = Cx<double>;
-    using G = LineGeo<L>;
+    using G = LineGeo<L, 16>;
     constexpr int M = G::M;
     __shared__ __align__(16) C xbuf[G::LINES][G::BUF + 1];
     const int li = threadIdx.x % G::LINES, a = threadIdx.x / G::LINES;
@@ -732,17 +732,17 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_dct_lines_reg(const double* 
     C v[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        const int e = a + 8 * m;
+        const int e = a + G::TL * m;
         const long long src = e <= L / 2 ? e : L - e;  // the even extension
         const double re = b0 < nb ? in[(long long)b0 * sb + obase + src * se] : 0.0;
         const double im = b1 < nb ? in[(long long)b1 * sb + obase + src * se] : 0.0;
         v[m] = C{re, im};
     }
-    line_fft<double, false, false, L, true>(v, a, xbuf[li], reinterpret_cast<const C*>(twd));
+    line_fft<double, false, false, L, true, 16>(v, a, xbuf[li], reinterpret_cast<const C*>(twd));
     if (b0 >= nb) return;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        const int e = a + 8 * m;
+        const int e = a + G::TL * m;
         if (e < len) {
             out[(long long)b0 * sb + obase + (long long)e * se] = (TO)v[m].x;
             if (b1 < nb) out[(long long)b1 * sb + obase + (long long)e * se] = (TO)v[m].y;
@@ -1032,10 +1032,14 @@ struct LaunchDct {
     void run() {
         // 256-point lines only: at 128 points the staged tiles measured faster
         // (Green's-function phase 41.6 against 45.6 us at 64^3), at 256 points
-        // the line form (185 against 175 us at 128^3)
+        // the line form (185 against 175 us at 128^3).  16 threads per line
+        // with 16 elements each, 16 warps per SM, took it from 138 to 128 us
+        // (phase profile; mixed 129 to 120); 8 threads held 32 in some 200 registers, 8 warps.
+        // The convolution's passes keep 8: with 16 their transforms of both
+        // types spill at 4 blocks and lose at 3 (156 -> 167 us at 128^3).
         if constexpr (!FROM_TMP && LT == 256) {
             if (register_lines() && pl.L == LT && len == LT / 2 + 1) {
-                using G = LineGeo<LT>;
+                using G = LineGeo<LT, 16>;
                 const int pairs = (nb + 1) / 2;
                 dim3 g((unsigned)((pairs + G::LINES - 1) / G::LINES), (unsigned)outer);
                 k_dct_lines_reg<TO, LT><<<g, G::NT, 0, s>>>(in, out, len, nb, sb, so, se, tw);

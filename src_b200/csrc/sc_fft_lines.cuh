@@ -177,17 +177,21 @@ __device__ __forceinline__ void dft_half(Cx<T>* v) {
 // A 32-point line (plan 4 8) has 4 threads, thread a the elements a + 4m:
 // the inputs of the first stage's butterflies a and a + 4, whose outputs go
 // through the exchange to the single radix-8 butterfly a of the last stage.
-template <int L>
+//
+// With 16 threads (256 points: k_dct_lines_reg) thread a holds the elements
+// a + 16m: the inputs of four butterflies of the first stage, exchanged those
+// of two of the second, exchanged again those of two of the last.
+template <int L, int T = L == 32 ? 4 : 8>
 struct LineGeo {
-    static constexpr int TL = L == 32 ? 4 : 8;  // threads per line
-    static constexpr int M = L / TL;            // elements per thread
-    static constexpr int BUF = L + 8;         // exchange buffer elements of a line
-    static constexpr int LINES = L >= 256 ? 8 : 16;  // lines per block
+    static constexpr int TL = T;      // threads per line
+    static constexpr int M = L / TL;  // elements per thread
+    static constexpr int BUF = TL == 16 ? L + L / 8 : L + 8;  // exchange buffer elements of a line
+    static constexpr int LINES = L >= 256 ? 8 : 16;           // lines per block
     static constexpr int NT = TL * LINES;
 };
-template <int L>
+template <int L, int TL = LineGeo<L>::TL>
 __device__ __forceinline__ int xidx(int p) {
-    return p + p / (L == 32 ? 8 : L / 8);
+    return p + p / (L == 32 || TL == 16 ? 8 : L / 8);
 }
 
 // What the exchange waits for: 0 the warp (the threads of a line are
@@ -204,10 +208,10 @@ __device__ __forceinline__ void line_sync() {
         asm volatile("bar.sync 1, %0;" ::"n"(SYNC) : "memory");
 }
 
-template <typename T, bool INV, bool HALF_IN, int L, int SYNC = 0>
-__device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L>::M], int a, Cx<T>* xs, const Cx<T>* __restrict__ tw) {
+template <typename T, bool INV, bool HALF_IN, int L, int SYNC = 0, int TL = LineGeo<L>::TL>
+__device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L, TL>::M], int a, Cx<T>* xs, const Cx<T>* __restrict__ tw) {
     using C = Cx<T>;
-    constexpr int M = LineGeo<L>::M;
+    constexpr int M = LineGeo<L, TL>::M;
     if constexpr (L == 32) {
         // stage 1: radix 4, Ns = 1; butterfly a + 4q reads elements a + 4q + 8r, writes 4 (a + 4q) + r
 #pragma unroll
@@ -218,13 +222,13 @@ __device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L>::M], int a, Cx<T>
             else
                 dft<T, 4, INV>(u);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) xs[xidx<L>(4 * (a + 4 * q) + r)] = u[r];
+            for (int r = 0; r < 4; ++r) xs[xidx<L, TL>(4 * (a + 4 * q) + r)] = u[r];
         }
         line_sync<SYNC>();
         // last stage: radix 8, Ns = 4, step 1; butterfly a reads and writes elements a + 4r
         C u[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L>(a + 4 * r)];
+        for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L, TL>(a + 4 * r)];
 #pragma unroll
         for (int r = 1; r < 8; ++r) {
             C t = __ldg(&tw[r * a]);
@@ -234,6 +238,60 @@ __device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L>::M], int a, Cx<T>
         dft<T, 8, INV>(u);
 #pragma unroll
         for (int r = 0; r < 8; ++r) v[r] = u[r];
+        line_sync<SYNC>();
+    } else if constexpr (TL == 16) {
+        // stage 1: radix 4, Ns = 1; butterfly j = a + 16q reads elements j + 64r, writes 4j + r
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            C u[4] = {v[q], v[q + 4], v[q + 8], v[q + 12]};
+            if constexpr (HALF_IN)
+                dft_half<T, 4, INV>(u);
+            else
+                dft<T, 4, INV>(u);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) xs[xidx<L, TL>(4 * (a + 16 * q) + r)] = u[r];
+        }
+        line_sync<SYNC>();
+        // stage 2: radix 8, Ns = 4, step 8; butterfly j = a + 16q reads elements j + 32r and
+        // writes 32 (j / 4) + j % 4 + 4r, once every butterfly of the line has read
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            C u[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L, TL>(a + 16 * q + 32 * r)];
+#pragma unroll
+            for (int r = 1; r < 8; ++r) {
+                C t = __ldg(&tw[r * (a % 4) * 8]);
+                if (INV) t.y = -t.y;
+                u[r] = cmul(u[r], t);
+            }
+            dft<T, 8, INV>(u);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[q + 2 * r] = u[r];
+        }
+        line_sync<SYNC>();
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int r = 0; r < 8; ++r) xs[xidx<L, TL>((a + 16 * q) / 4 * 32 + a % 4 + 4 * r)] = v[q + 2 * r];
+        line_sync<SYNC>();
+        // last stage: radix 8, Ns = 32, step 1; butterfly j = a + 16q reads and writes elements j + 32r
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int j = a + 16 * q;
+            C u[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L, TL>(j + 32 * r)];
+#pragma unroll
+            for (int r = 1; r < 8; ++r) {
+                C t = __ldg(&tw[r * j]);
+                if (INV) t.y = -t.y;
+                u[r] = cmul(u[r], t);
+            }
+            dft<T, 8, INV>(u);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[q + 2 * r] = u[r];
+        }
         line_sync<SYNC>();
     } else {
         C o[M];  // elements M a + i after the stages before the exchange
@@ -288,7 +346,7 @@ __device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L>::M], int a, Cx<T>
             }
         }
 #pragma unroll
-        for (int i = 0; i < M; ++i) xs[xidx<L>(M * a + i)] = o[i];
+        for (int i = 0; i < M; ++i) xs[xidx<L, TL>(M * a + i)] = o[i];
         line_sync<SYNC>();
         // last stage: radix 8, Ns = M, step 1; butterfly j = a + 8s reads
         // elements j + M r and writes them back in place
@@ -297,7 +355,7 @@ __device__ __forceinline__ void line_fft(Cx<T> (&v)[LineGeo<L>::M], int a, Cx<T>
             const int j = a + 8 * s2;
             C u[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L>(j + M * r)];
+            for (int r = 0; r < 8; ++r) u[r] = xs[xidx<L, TL>(j + M * r)];
 #pragma unroll
             for (int r = 1; r < 8; ++r) {
                 C t = __ldg(&tw[r * j]);
