@@ -995,6 +995,11 @@ struct LaunchRfftNeg {
     }
 };
 
+// Pass E's threads: staging, packing and scaling its tile take more of them
+// than its butterflies need, so no fewer than 256 up to 128 points (48^3 step
+// 78.6 -> 76.8 us, 64^3 131.8 -> 129.9).  At 256 points fewer blocks fit and
+// it loses (128^3 convolution 156 -> 159.5 us).
+__host__ __device__ constexpr int threads_e(int lt, int nt) { return lt > 0 && lt <= 128 && nt < 256 ? 256 : nt; }
 template <bool SELF, bool FLIP = false, bool FULL = false>
 struct LaunchE {
     const double2* spec;
@@ -1011,7 +1016,7 @@ struct LaunchE {
     }
     template <int LT, int V>
     void go() {
-        constexpr int NC = Geo<LT, V>::NC, NT = Geo<LT, V>::NT;
+        constexpr int NC = Geo<LT, V>::NC, NT = threads_e(LT, Geo<LT, V>::NT);
         dim3 g((unsigned)((n0 + 2 * NC - 1) / (2 * NC)), (unsigned)n1);
         k_fft_z_c2r<double, SELF, LT, NC, NT, FLIP, FULL><<<g, NT, smem_of<double2>(pz.L, NC), s>>>(
             spec, phi, n0, n1, n2, L0, L1, pz, twz, st, normFact, coupling);
@@ -1084,23 +1089,23 @@ struct SetLimits {
         allow(k_fft_y<double, true, LT, NC, NT>);
         allow(k_fft_x_conv<double, double, LT, NC, NT>);
         allow(k_fft_x_conv<float, double, LT, NC, NT>);
-        allow(k_fft_z_c2r<double, true, LT, NC, NT>);
-        allow(k_fft_z_c2r<double, false, LT, NC, NT>);
+        allow(k_fft_z_c2r<double, true, LT, NC, threads_e(LT, NT)>);
+        allow(k_fft_z_c2r<double, false, LT, NC, threads_e(LT, NT)>);
         allow(k_dct_lines<double, LT, NC, NT>);
         allow(k_dct_lines<float, LT, NC, NT>);
         allow(k_dct_lines<double, LT, NC, 256, true>);
         allow(k_fft_x_conv<double, double, LT, NC, NT, true>);
         allow(k_fft_x_conv<float, double, LT, NC, NT, true>);
-        allow(k_fft_z_c2r<double, true, LT, NC, NT, true>);
-        allow(k_fft_z_c2r<double, false, LT, NC, NT, true>);
+        allow(k_fft_z_c2r<double, true, LT, NC, threads_e(LT, NT), true>);
+        allow(k_fft_z_c2r<double, false, LT, NC, threads_e(LT, NT), true>);
         allow(k_rfft_lines_neg<double, LT, NC, NT>);
         allow(k_rfft_lines_neg<float, LT, NC, NT>);
         allow(k_rfft_lines_neg<double, LT, NC, NT, false>);
         allow(k_rfft_lines_neg<float, LT, NC, NT, false>);
         allow(k_fft_z_r2c<double, LT, NC, NT, true>);
         allow(k_fft_z_r2c<float, LT, NC, NT, true>);
-        allow(k_fft_z_c2r<double, true, LT, NC, NT, false, true>);
-        allow(k_fft_z_c2r<double, false, LT, NC, NT, false, true>);
+        allow(k_fft_z_c2r<double, true, LT, NC, threads_e(LT, NT), false, true>);
+        allow(k_fft_z_c2r<double, false, LT, NC, threads_e(LT, NT), false, true>);
     }
 };
 
