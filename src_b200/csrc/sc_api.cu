@@ -269,6 +269,14 @@ DevBunch bin_view(const scgpu_ctx* c, int k) {
 
 void enqueue_reorder_beside(scgpu_ctx* c, cudaEvent_t after);
 
+// The charge density and the forward transforms, which pass A starts from the
+// accumulators where it can.
+void enqueue_assemble_forward(const DevBunch& b, cudaStream_t s) {
+    const bool fused = fft_assembles(b);
+    if (!fused) launch_assemble_rho(b, s);
+    launch_convolution_part(b, kConvSelfField, kConvForwardPart | (fused ? kConvAssemble : 0), s);
+}
+
 // The energy-bin loop of computeSpaceChargeFields (ParallelTTracker.cpp:567-578)
 // once the drift kernel has set this step's mesh: calcGammas, one deposit pass
 // for all active bins, then per bin the charge density, the bin's own
@@ -297,8 +305,7 @@ void enqueue_bins_fields(scgpu_ctx* c, bool reorder, cudaStream_t s) {
         launch_igf_image(v, c->side);
         launch_green_transform_image(v, c->side);
         cudaEventRecord(c->ev_bin[k], c->side);
-        launch_assemble_rho(v, s);
-        launch_convolution_part(v, kConvSelfField, kConvForwardPart, s);
+        enqueue_assemble_forward(v, s);
         cudaStreamWaitEvent(s, c->ev_bin[k], 0);
         launch_convolution_part(v, kConvSelfField, kConvRestPart, s);
         DevBunch vi = v;  // the image's potential into its own buffer
@@ -431,8 +438,7 @@ void enqueue_step(scgpu_ctx* c, bool stats, bool reorder, cudaStream_t s) {
     }
     if (shard)  // the charge of all shards: exact integer node sums
         exchange(c, b.nacc, 2 * mesh_cells(b), SCGPU_EXCHANGE_SUM_U64, s);
-    launch_assemble_rho(b, s);
-    launch_convolution_part(b, kConvSelfField, kConvForwardPart, s);
+    enqueue_assemble_forward(b, s);
     cudaStreamWaitEvent(s, c->ev_join, 0);
     launch_convolution_part(b, kConvSelfField, kConvRestPart, s);
     launch_grad(b, s);
@@ -1158,8 +1164,7 @@ int scgpu_compute_self_fields(scgpu_ctx* c, long long n, const double* R, const 
     fork_green(c, false, s);
     launch_deposit(b, s);
     STAGE("deposit");
-    launch_assemble_rho(b, s);
-    launch_convolution_part(b, kConvSelfField, kConvForwardPart, s);
+    enqueue_assemble_forward(b, s);
     STAGE("assemble");
     CK(cudaStreamWaitEvent(s, c->ev_join, 0));
     launch_convolution_part(b, kConvSelfField, kConvRestPart, s);

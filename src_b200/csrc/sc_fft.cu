@@ -34,6 +34,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "sc_exact.cuh"
 #include "sc_fft_lines.cuh"
 
 namespace sc {
@@ -531,10 +532,21 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_y_lines(Cx<T>* __restric
 // column pairs, so a warp reads and writes whole rows) and block-level
 // exchanges.  The two half spectra need Z[k] and Z[L - k], which sit in
 // different threads: the transformed line goes through its buffer once more.
-template <typename T, int L>
-__global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_z_r2c_lines(const T* __restrict__ rho, Cx<T>* __restrict__ spec,
+//
+// ACC: the charge density is formed here from the deposit's accumulators
+// (k_assemble_rho: the same values, rho stored, the accumulators cleared), which
+// saves a launch of the small meshes where launches are what the step waits
+// for (fft_assembles).
+struct AccIn {
+    ulonglong2* acc;
+    const StepState* st;
+    double dT, rdT;
+    int weights;
+};
+template <typename T, int L, bool ACC = false>
+__global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_z_r2c_lines(T* __restrict__ rho, Cx<T>* __restrict__ spec,
                                                                   int n0, int n1, int L0, int L1,
-                                                                  const Cx<T>* __restrict__ twz) {
+                                                                  const Cx<T>* __restrict__ twz, AccIn in) {
     using C = Cx<T>;
     using G = LineGeo<L>;
     constexpr int M = G::M, K = L / 2;
@@ -546,13 +558,29 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_z_r2c_lines(const T* __r
     const bool live = y < n1;
     const bool odd = live && x + 1 < n0;
     C v[M];
+    double unit = 0.0, tmp2 = 0.0;
+    if constexpr (ACC) {
+        unit = in.weights ? in.st->qdt * 0x1p-26 : in.st->dep_unit;
+        tmp2 = in.st->tmp2;
+    }
 #pragma unroll
     for (int m = 0; m < M; ++m) {
         v[m] = C{(T)0, (T)0};
         if (live && m < M / 2) {
-            const T* p = rho + ((size_t)(a + G::TL * m) * n1 + y) * n0 + x;
-            v[m].x = p[0];
-            if (odd) v[m].y = p[1];
+            const size_t c = ((size_t)(a + G::TL * m) * n1 + y) * n0 + x;
+            if constexpr (ACC) {
+                v[m].x = (T)node_density(in.acc[c], unit, in.dT, in.rdT, tmp2);
+                rho[c] = v[m].x;
+                in.acc[c] = make_ulonglong2(0ull, 0ull);
+                if (odd) {
+                    v[m].y = (T)node_density(in.acc[c + 1], unit, in.dT, in.rdT, tmp2);
+                    rho[c + 1] = v[m].y;
+                    in.acc[c + 1] = make_ulonglong2(0ull, 0ull);
+                }
+            } else {
+                v[m].x = rho[c];
+                if (odd) v[m].y = rho[c + 1];
+            }
         }
     }
     C* xs = xbuf[li];
@@ -841,8 +869,8 @@ int single_variant(int LT) {
     return LT >= 64 ? 1 : 0;  // half-width tiles measured faster from 64 points up (the cosine transforms most)
 }
 
-// Passes A (open z), B, C and D of 64-, 128- and 256-point lines take the
-// register-resident kernels (k_*_lines, the same bits as the staged ones);
+// Passes A (open z; from 32 points), B, C and D of 64-, 128- and 256-point
+// lines take the register-resident kernels (k_*_lines, the same bits as the staged ones);
 // pass E stays staged (its line form measured slower: 10.1 against 7.0 us
 // at 128 points, 32.6 against 26.2 us at 256).  SCGPU_FFT_LINES=0 selects
 // the staged kernels everywhere.
@@ -888,22 +916,32 @@ void with_length(int L, F&& f) {
     }
 }
 
+// The longest z transform whose pass A can form rho itself (fft_assembles).
+constexpr int kAssembleMax = 64;
+
 template <typename T, bool FULL = false>
 struct LaunchA {
-    const T* rho;
+    T* rho;
     Cx<T>* spec;
     int n0, n1, n2, L0, L1;
     FftPlan pz;
     const Cx<T>* twz;
     cudaStream_t s;
+    const AccIn* in = nullptr;  // form rho from the accumulators (fft_assembles)
     template <int LT>
     void run() {
-        if constexpr (!FULL && (LT == 64 || LT == 128 || LT == 256)) {
+        if constexpr (!FULL && (LT == 32 || LT == 64 || LT == 128 || LT == 256)) {
             if (register_lines() && 2 * n2 == LT) {
                 using G = LineGeo<LT>;
                 const long long lines = (long long)n1 * ((n0 + 1) / 2);
-                k_fft_z_r2c_lines<T, LT><<<(unsigned)((lines + G::LINES - 1) / G::LINES), G::NT, 0, s>>>(
-                    rho, spec, n0, n1, L0, L1, twz);
+                const unsigned g = (unsigned)((lines + G::LINES - 1) / G::LINES);
+                if constexpr (LT <= kAssembleMax) {
+                    if (in) {
+                        k_fft_z_r2c_lines<T, LT, true><<<g, G::NT, 0, s>>>(rho, spec, n0, n1, L0, L1, twz, *in);
+                        return;
+                    }
+                }
+                k_fft_z_r2c_lines<T, LT><<<g, G::NT, 0, s>>>(rho, spec, n0, n1, L0, L1, twz, AccIn{});
                 return;
             }
         }
@@ -1276,6 +1314,16 @@ inline bool special_length(int L) { return L == 32 || L == 64 || L == 96 || L ==
 
 bool fft_register_lines() { return register_lines(); }
 
+// Up to 40^3 cells the step waits on its launches, and the separate assembly
+// is one (32^3, 1e5 particles: 51.0 -> 48.0 us a step, mixed 47.7 -> 45.5); at
+// 64^3 the assembly fills the GPU and does its divisions faster than the
+// transform's threads between their loads (mixed 107.5 against 109.2 us).
+bool fft_assembles(const DevBunch& b) {
+    const int L2 = 2 * b.bc.n[2];
+    return register_lines() && !b.periodic_z && (L2 == 32 || L2 == kAssembleMax) &&
+           (long long)b.bc.n[0] * b.bc.n[1] * b.bc.n[2] <= 64000;
+}
+
 bool fft_pass_plane(const DevBunch& b, int variant) {
     return variant == kFftLinesVariant && fft_plane_length(2 * b.bc.n[0], 2 * b.bc.n[1]);
 }
@@ -1543,10 +1591,12 @@ static void convolution_t(const DevBunch& b, int mode, int parts, cudaStream_t s
     normFact /= L1;
     normFact /= L2;
     if (parts & kConvForwardPart) {
+        const AccIn acc{reinterpret_cast<ulonglong2*>(b.nacc), b.st, b.bc.dT, b.bc.rdT, b.dep_weights};
         if (b.periodic_z)
-            with_length(L2, LaunchA<T, true>{(const T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s});
+            with_length(L2, LaunchA<T, true>{(T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s});
         else
-            with_length(L2, LaunchA<T>{(const T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s});
+            with_length(L2, LaunchA<T>{(T*)b.rho, fwd, n0, n1, n2, L0, L1, pz, twz, s,
+                                       (parts & kConvAssemble) ? &acc : nullptr});
         if (!plane) with_length(L1, LaunchY<T, false>{fwd, n0, L0, n1, L1, K + 1, py, twy, s});
     }
     // passes C and D, or B, C and D of a plane in one kernel

@@ -259,7 +259,10 @@ void launch_convolution(const DevBunch& b, int mode, cudaStream_t s);
 // the forward passes (A, B) need rho only; the rest (C, D, E) also the spectrum of G.
 // The image part runs C, D, E with the shifted G's complex spectrum and
 // writes phi with z flipped (FFTPoissonSolver.cpp:312-326).
-enum : int { kConvForwardPart = 1, kConvRestPart = 2, kConvImagePart = 4 };
+// kConvAssemble: pass A forms rho from the deposit's accumulators, as
+// launch_assemble_rho (only where fft_assembles).
+enum : int { kConvForwardPart = 1, kConvRestPart = 2, kConvImagePart = 4, kConvAssemble = 8 };
+bool fft_assembles(const DevBunch& b);
 void launch_convolution_part(const DevBunch& b, int mode, int parts, cudaStream_t s);
 // spectrum of the shifted G (b.gimg) into b.ghat_img
 void launch_green_transform_image(const DevBunch& b, cudaStream_t s);
