@@ -496,11 +496,19 @@ __global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_x_conv_lines(const Cx<TI
 // Passes B (forward, inputs y < L/2) and D (inverse, outputs y < L/2) on
 // columns of L points along y: TL threads per column (in different warps),
 // consecutive x of one plane per block.
+// FP64 columns of 256 points take 16 threads of 128 registers: with 8 of 186
+// pass D had 7 warps per SM waiting for its columns (issue 16 %).  128^3 step
+// 903 -> 901 us, mixed 702 -> 694.
+template <typename T, int L>
+using YGeo = LineGeo<L, L == 256 && sizeof(T) == sizeof(double) ? 16 : LineGeo<L>::TL>;
+template <typename T, int L>
+constexpr int kYBlocks = YGeo<T, L>::TL == 16 ? 4 : 1;  // 128 registers with 16 threads per line
+
 template <typename T, bool INV, int L>
 __device__ __forceinline__ void fft_y_lines_body(Cx<T>* __restrict__ spec, int n0, int L0, int planes,
                                                  const Cx<T>* __restrict__ twy, int bx, int kz) {
     using C = Cx<T>;
-    using G = LineGeo<L>;
+    using G = YGeo<T, L>;
     constexpr int M = G::M;
     // lanes run along x (thread li + LINES a: column li, part a), so a warp
     // reads and writes whole rows of consecutive columns; the line buffers
@@ -509,20 +517,21 @@ __device__ __forceinline__ void fft_y_lines_body(Cx<T>* __restrict__ spec, int n
     const int li = threadIdx.x % G::LINES, a = threadIdx.x / G::LINES;
     const int x = bx * G::LINES + li;
     const bool live = kz < planes && x < n0;
-    C* col = spec + (size_t)kz * L * L0 + (live ? x : 0);
+    C* col = spec + ((size_t)kz * L + a) * L0 + (live ? x : 0);
+    const unsigned step = (unsigned)(G::TL * L0);
     C v[M];
 #pragma unroll
     for (int m = 0; m < M; ++m)
-        v[m] = (live && (INV || m < M / 2)) ? col[(size_t)(a + G::TL * m) * L0] : C{(T)0, (T)0};
-    line_fft<T, INV, !INV, L, true>(v, a, xbuf[li], twy);
+        v[m] = (live && (INV || m < M / 2)) ? col[(unsigned)m * step] : C{(T)0, (T)0};
+    line_fft<T, INV, !INV, L, true, G::TL>(v, a, xbuf[li], twy);
     if (!live) return;
     constexpr int MO = INV ? M / 2 : M;  // D keeps y < L/2
 #pragma unroll
-    for (int m = 0; m < MO; ++m) col[(size_t)(a + G::TL * m) * L0] = v[m];
+    for (int m = 0; m < MO; ++m) col[(unsigned)m * step] = v[m];
 }
 
 template <typename T, bool INV, int L>
-__global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_y_lines(Cx<T>* __restrict__ spec, int n0, int L0, int planes,
+__global__ void __launch_bounds__(YGeo<T, L>::NT, kYBlocks<T, L>) k_fft_y_lines(Cx<T>* __restrict__ spec, int n0, int L0, int planes,
                                                               const Cx<T>* __restrict__ twy) {
     fft_y_lines_body<T, INV, L>(spec, n0, L0, planes, twy, blockIdx.x, blockIdx.y);
 }
@@ -870,10 +879,9 @@ int single_variant(int LT) {
 }
 
 // Passes A (open z; from 32 points), B, C and D of 64-, 128- and 256-point
-// lines take the register-resident kernels (k_*_lines, the same bits as the staged ones);
-// pass E stays staged (its line form measured slower: 10.1 against 7.0 us
-// at 128 points, 32.6 against 26.2 us at 256).  SCGPU_FFT_LINES=0 selects
-// the staged kernels everywhere.
+// lines take the register-resident kernels (k_*_lines, the same bits as the
+// staged ones); pass E stays staged.  SCGPU_FFT_LINES=0 selects the staged
+// kernels everywhere.
 bool register_lines() {
     static const bool on = [] {
         const char* e = std::getenv("SCGPU_FFT_LINES");
@@ -966,7 +974,7 @@ struct LaunchY {
     void run() {
         if constexpr (LT == 64 || LT == 128 || LT == 256) {
             if (register_lines() && 2 * (INV ? n_out : n_in) == LT) {
-                using G = LineGeo<LT>;
+                using G = YGeo<T, LT>;
                 const dim3 g((unsigned)((n0 + G::LINES - 1) / G::LINES), (unsigned)planes);
                 k_fft_y_lines<T, INV, LT><<<g, G::NT, 0, s>>>(spec, n0, L0, planes, twy);
                 return;
@@ -1033,10 +1041,9 @@ struct LaunchRfftNeg {
     }
 };
 
-// Pass E's threads: staging, packing and scaling its tile take more of them
-// than its butterflies need, so no fewer than 256 up to 128 points (48^3 step
-// 78.6 -> 76.8 us, 64^3 131.8 -> 129.9).  At 256 points fewer blocks fit and
-// it loses (128^3 convolution 156 -> 159.5 us).
+// Threads of the staged pass E: staging, packing and scaling its tile take more
+// of them than its butterflies need, so no fewer than 256 up to 128 points
+// (48^3 step 78.6 -> 76.8 us).  At 256 points fewer blocks fit and it loses.
 __host__ __device__ constexpr int threads_e(int lt, int nt) { return lt > 0 && lt <= 128 && nt < 256 ? 256 : nt; }
 template <bool SELF, bool FLIP = false, bool FULL = false>
 struct LaunchE {
@@ -1218,7 +1225,13 @@ inline bool line_length(int L) { return L == 64 || L == 128 || L == 256; }
 // lines run the register-resident line transforms (the same bits), block
 // (x, y) of a bunch as in the single-bunch launch.
 template <typename T, int PASS, int L>
-__global__ void __launch_bounds__(LineGeo<L>::NT) k_fft_lines_batch(const DevBunch* __restrict__ tab,
+struct BatchLines {
+    using TY = typename std::conditional<PASS == kPassYInv, double, T>::type;
+    static constexpr int NT = PASS == kPassXConv ? LineGeo<L>::NT : YGeo<TY, L>::NT;
+    static constexpr int MINB = PASS == kPassXConv ? 1 : kYBlocks<TY, L>;
+};
+template <typename T, int PASS, int L>
+__global__ void __launch_bounds__(BatchLines<T, PASS, L>::NT, BatchLines<T, PASS, L>::MINB) k_fft_lines_batch(const DevBunch* __restrict__ tab,
                                                                   const int4* __restrict__ work, int nitems) {
     const int4 w = resolve_block(work, nitems);
     const DevBunch& d = tab[w.x];
@@ -1244,7 +1257,7 @@ struct LaunchLinesBatch {
     template <int LT>
     void run() {
         if constexpr (LT == 64 || LT == 128 || LT == 256)
-            k_fft_lines_batch<T, PASS, LT><<<n, LineGeo<LT>::NT, 0, s>>>(tab, work, nitems);
+            k_fft_lines_batch<T, PASS, LT><<<n, BatchLines<T, PASS, LT>::NT, 0, s>>>(tab, work, nitems);
     }
 };
 
