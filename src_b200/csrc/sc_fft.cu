@@ -787,6 +787,99 @@ __global__ void __launch_bounds__(LineGeo<L, 16>::NT, 4) k_dct_lines_reg(const d
     }
 }
 
+// The first cosine transform (z lines of one y) with G formed in registers:
+// TL threads per pair of lines (b0 = 2p, b0 + 1), lanes along p.  Thread a
+// forms the L/(2 TL) consecutive elements of its part of both lines, so one
+// plane of the antiderivative (3 x by 2 y values) serves two elements in z and
+// the shared column two in x: 3.4 loads per element in place of igf_G_at's 8,
+// in whole rows; the elements and their mirrors then go through the line's
+// buffer to the transform's order.  Same operation order as igf_G_at.  The
+// staged form (dct_lines_body<FROM_TMP>) reads 32-byte pieces of eight planes
+// per access, 83 % of the L1 throughput at 256 points.  Green's-function phase,
+// staged -> this: 128^3 128.7 -> 114.8 us (mixed 120.4 -> 106.7), 64^3 36.0 ->
+// 33.8 (31.9 -> 29.8).  At 32 and 64 points the branch gains 1 us at most, the
+// step nothing (32^3 slower: 49.7 -> 56 us), and the staged form stays.
+template <int L>
+using ZLine = LineGeo<L, L == 256 ? 16 : 8>;
+template <int L>
+struct ZGeo {
+    using G = ZLine<L>;
+    static constexpr int TL = G::TL, LINES = 8, NT = TL * LINES;
+};
+template <int L>
+__global__ void __launch_bounds__(ZGeo<L>::NT, 512 / ZGeo<L>::NT) k_dct_z_lines(const double* __restrict__ tmp,
+                                                                                double* __restrict__ out, int nb,
+                                                                                long long so, long long se,
+                                                                                const double2* __restrict__ twd, int t0,
+                                                                                int t1) {
+    using G = typename ZGeo<L>::G;
+    constexpr int N = L / 2, M = G::M, TL = G::TL, LINES = ZGeo<L>::LINES, CH = N / TL;
+    __shared__ __align__(16) double2 xbuf[LINES][G::BUF + 1];
+    const int li = threadIdx.x % LINES, a = threadIdx.x / LINES;
+    const int b0 = 2 * (blockIdx.x * LINES + li), j = blockIdx.y;
+    const bool one = b0 < nb, two = b0 + 1 < nb;
+    double2* xs = xbuf[li];
+    const long long plane = (long long)t0 * t1;
+    const double* q = tmp + (one ? b0 : 0) + (long long)j * t0 + (long long)(a * CH) * plane;
+    // c: the values at (b0 .. b0 + 2, j) and (.., j + 1) of plane k, d: of plane k + 1
+    double c[6], d[6];
+    auto load = [&](double* v, const double* r) {
+        v[0] = r[0];
+        v[1] = r[1];
+        v[2] = two ? r[2] : 0.0;
+        v[3] = r[t0];
+        v[4] = r[t0 + 1];
+        v[5] = two ? r[t0 + 2] : 0.0;
+    };
+    auto corner = [&](int i) {
+        double g = d[i + 4];
+        g += c[i + 1];
+        g += c[i + 3];
+        g += d[i];
+        g -= c[i + 4];
+        g -= d[i + 1];
+        g -= d[i + 3];
+        g -= c[i];
+        return g;
+    };
+    load(c, q);
+    double2 first{0.0, 0.0};
+    const int cnt = a == TL - 1 ? CH + 1 : CH;  // the last thread also forms element N
+#pragma unroll
+    for (int m = 0; m <= CH; ++m) {
+        if (m < cnt) {
+            load(d, q + (long long)(m + 1) * plane);
+            double2 g{one ? corner(0) : 0.0, two ? corner(1) : 0.0};
+            if (m == 0) first = g;
+            // G[0,0,0] <- G[0,0,1]
+            if (m == 1 && a == 0) xs[xidx<L, TL>(0)] = double2{b0 == 0 && j == 0 ? g.x : first.x, first.y};
+            const int e = a * CH + m;
+            if (e > 0) {
+                xs[xidx<L, TL>(e)] = g;
+                if (e < N) xs[xidx<L, TL>(L - e)] = g;
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) c[k] = d[k];
+        }
+    }
+    __syncthreads();
+    double2 v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = xs[xidx<L, TL>(a + TL * m)];
+    __syncthreads();
+    line_fft<double, false, false, L, 1, TL>(v, a, xs, twd);
+    if (!one) return;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const int e = a + TL * m;
+        if (e <= N) {
+            double* o = out + b0 + (long long)j * so + (long long)e * se;
+            o[0] = v[m].x;
+            if (two) o[1] = v[m].y;
+        }
+    }
+}
+
 // Full real transform of lines of length L along z (stride se), 2 NC lines
 // per block packed two per complex FFT and split by the Hermitian symmetry,
 // as pass A; the half spectrum k in [0, L/2] of line b goes to
@@ -879,9 +972,10 @@ int single_variant(int LT) {
 }
 
 // Passes A (open z; from 32 points), B, C and D of 64-, 128- and 256-point
-// lines take the register-resident kernels (k_*_lines, the same bits as the
-// staged ones); pass E stays staged.  SCGPU_FFT_LINES=0 selects the staged
-// kernels everywhere.
+// lines and G's z transform of 128- and 256-point lines take the
+// register-resident kernels (k_*_lines, the same bits as the staged ones); pass
+// E stays staged.
+// SCGPU_FFT_LINES=0 selects the staged kernels everywhere.
 bool register_lines() {
     static const bool on = [] {
         const char* e = std::getenv("SCGPU_FFT_LINES");
@@ -1093,6 +1187,14 @@ struct LaunchDct {
                 const int pairs = (nb + 1) / 2;
                 dim3 g((unsigned)((pairs + G::LINES - 1) / G::LINES), (unsigned)outer);
                 k_dct_lines_reg<TO, LT><<<g, G::NT, 0, s>>>(in, out, len, nb, sb, so, se, tw);
+                return;
+            }
+        }
+        if constexpr (FROM_TMP && (LT == 128 || LT == 256)) {
+            if (register_lines() && pl.L == LT && len == LT / 2 + 1 && sb == 1) {
+                using Z = ZGeo<LT>;
+                dim3 g((unsigned)(((nb + 1) / 2 + Z::LINES - 1) / Z::LINES), (unsigned)outer);
+                k_dct_z_lines<LT><<<g, Z::NT, 0, s>>>(in, out, nb, so, se, tw, t0, t1);
                 return;
             }
         }
