@@ -686,6 +686,66 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_fft_z_c2r(const Cx<T>* __rest
                                                     blockIdx.x, blockIdx.y);
 }
 
+// Pass E on z lines of L = 2 n2 points (as k_fft_z_r2c_lines backwards): two
+// half spectra (x, x + 1) of one y per complex line, lanes along x; thread a
+// packs the elements k = a + TL m <= L/2 and their mirrors through the line's
+// buffer, so each spectrum entry is read once.  The staged form moves the tile
+// through shared memory at every stage (75 % of the L1 throughput at 256
+// points).  Convolution phase, staged -> this: 128^3 152.3 -> 143.0 us (mixed
+// 133.6 -> 122.9), 64^3 32.8 -> 31.8 (29.8 -> 28.7).  At 32 and 64 points the
+// step does not move and the staged form stays.
+template <int L>
+using ZLine = LineGeo<L, L == 256 ? 16 : 8>;
+template <bool SELF, int L, bool FLIP>
+__global__ void __launch_bounds__(ZLine<L>::NT, L == 256 ? 4 : 1)
+    k_fft_z_c2r_lines(const double2* __restrict__ spec, double* __restrict__ phi, int n0, int n1, int L0, int L1,
+                      const double2* __restrict__ twz, const StepState* __restrict__ st, double normFact,
+                      double coupling) {
+    using G = ZLine<L>;
+    constexpr int M = G::M, TL = G::TL, K = L / 2, LINES = G::LINES;
+    __shared__ __align__(16) double2 xbuf[LINES][G::BUF + 1];
+    const int li = threadIdx.x % LINES, a = threadIdx.x / LINES;
+    const int np = (n0 + 1) / 2;
+    const int line = blockIdx.x * LINES + li;
+    const int y = line / np, x = 2 * (line - y * np);
+    const bool live = y < n1;
+    const bool odd = live && x + 1 < n0;
+    double2* xs = xbuf[li];
+    const double2* src = spec + (live ? (size_t)y * L0 + x : 0);
+    const size_t plane = (size_t)L1 * L0;
+#pragma unroll
+    for (int m = 0; m <= M / 2; ++m) {
+        const int k = a + TL * m;
+        if (m < M / 2 || a == 0) {
+            double2 A = live ? src[k * plane] : double2{0.0, 0.0};
+            double2 B = odd ? src[k * plane + 1] : double2{0.0, 0.0};
+            if (k == 0 || k == K) A.y = B.y = 0.0;  // the half-complex format holds no imaginary part there
+            xs[xidx<L, TL>(k)] = double2{A.x - B.y, A.y + B.x};
+            if (k > 0 && k < K) xs[xidx<L, TL>(L - k)] = double2{A.x + B.y, B.x - A.y};
+        }
+    }
+    __syncthreads();
+    double2 v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = xs[xidx<L, TL>(a + TL * m)];
+    __syncthreads();
+    line_fft<double, true, false, L, 1, TL>(v, a, xs, twz);
+    if (!live) return;
+    const double hvol = SELF ? st->hvol : 1.0;
+#pragma unroll
+    for (int m = 0; m < M / 2; ++m) {
+        const int zz = a + TL * m;
+        double re = v[m].x * normFact, im = v[m].y * normFact;
+        if (SELF) {
+            re = re * hvol * coupling;
+            im = im * hvol * coupling;
+        }
+        double* o = phi + ((size_t)(FLIP ? K - 1 - zz : zz) * n1 + y) * n0 + x;
+        o[0] = re;
+        if (odd) o[1] = im;
+    }
+}
+
 // ---------------------------------------------------------------- G spectrum
 // Cosine transform of every line along one axis: Y[m] = sum over the even
 // extension (length L = 2(len-1)) of g, m in [0, len-1].  Lines are addressed
@@ -799,8 +859,6 @@ __global__ void __launch_bounds__(LineGeo<L, 16>::NT, 4) k_dct_lines_reg(const d
 // staged -> this: 128^3 128.7 -> 114.8 us (mixed 120.4 -> 106.7), 64^3 36.0 ->
 // 33.8 (31.9 -> 29.8).  At 32 and 64 points the branch gains 1 us at most, the
 // step nothing (32^3 slower: 49.7 -> 56 us), and the staged form stays.
-template <int L>
-using ZLine = LineGeo<L, L == 256 ? 16 : 8>;
 template <int L>
 struct ZGeo {
     using G = ZLine<L>;
@@ -972,9 +1030,8 @@ int single_variant(int LT) {
 }
 
 // Passes A (open z; from 32 points), B, C and D of 64-, 128- and 256-point
-// lines and G's z transform of 128- and 256-point lines take the
-// register-resident kernels (k_*_lines, the same bits as the staged ones); pass
-// E stays staged.
+// lines, E and G's z transform of 128- and 256-point lines take the
+// register-resident kernels (k_*_lines, the same bits as the staged ones).
 // SCGPU_FFT_LINES=0 selects the staged kernels everywhere.
 bool register_lines() {
     static const bool on = [] {
@@ -1151,6 +1208,15 @@ struct LaunchE {
     cudaStream_t s;
     template <int LT>
     void run() {
+        if constexpr (!FULL && (LT == 128 || LT == 256)) {
+            if (register_lines() && 2 * n2 == LT) {
+                using G = ZLine<LT>;
+                const int lines = n1 * ((n0 + 1) / 2);
+                k_fft_z_c2r_lines<SELF, LT, FLIP><<<(unsigned)((lines + G::LINES - 1) / G::LINES), G::NT, 0, s>>>(
+                    spec, phi, n0, n1, L0, L1, twz, st, normFact, coupling);
+                return;
+            }
+        }
         with_variant<LT>(*this);
     }
     template <int LT, int V>
