@@ -651,18 +651,6 @@ SC_HD void add_external_fields(const MapElem* el, int n, const Trafo& ref_to_lab
 }
 
 // ---------------------------------------------------------------- pusher
-// BorisPusher::push between switchToUnitlessPositions / switchOff...
-SC_HD void push_one(double* R, const double* P, double dt) {
-    const double s = kC * dt;
-    double r0 = R[0] / s, r1 = R[1] / s, r2 = R[2] / s;
-    double g = sqrt(1.0 + dot3(P, P));
-    r0 += 0.5 * P[0] / g;
-    r1 += 0.5 * P[1] / g;
-    r2 += 0.5 * P[2] / g;
-    R[0] = r0 * s;
-    R[1] = r1 * s;
-    R[2] = r2 * s;
-}
 // BorisPusher::kick
 SC_HD void kick_one(double* P, const double* Ef, const double* Bf, double dt, double mass, double charge) {
     const double ke = 0.5 * dt * charge * kC / mass;
@@ -825,8 +813,9 @@ SC_HD double wrap_z(double t, double lo, double hi) {
     return t;
 }
 
-// push_one in two parts: the unitless step 0.5 P / gamma, and R moved by it
-// (s = c dt, rs = RN(1/s) precomputed); together the same results.
+// BorisPusher::push between switchToUnitlessPositions and its way back, in two
+// parts: the unitless step 0.5 P / gamma, and R moved by it (s = c dt,
+// rs = RN(1/s) precomputed).
 SC_HD void push_step(const double* P, double* step) {
     bool fast = true;
     const double g = sqrt(1.0 + dot3(P, P));
