@@ -372,7 +372,10 @@ int scgpu_bunch_download(scgpu_ctx* ctx, double* R, double* P);
 /* Advance the device-resident bunch by nsteps ParallelTTracker steps.  When
  * stats is not NULL it receives nsteps records of SCGPU_NSTATS doubles: the
  * moment sums of the state at the end of each step (asynchronous copies;
- * pinned memory keeps them off the critical path). */
+ * pinned memory keeps them off the critical path).  A call that breaks off
+ * because CUDA refuses to build or launch a step graph leaves the bunch in
+ * the state after whole steps (scgpu_get_tracker_state counts them); where
+ * that is not certain it has to be uploaded again (SCGPU_ERR_STATE). */
 int scgpu_track(scgpu_ctx* ctx, int nsteps, double* stats);
 
 /* Energy bins of the resident bunch: bins[i] is the bin of particle i in the

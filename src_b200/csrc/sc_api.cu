@@ -70,6 +70,7 @@ int fail(scgpu_ctx* c, int code, const std::string& what) {
 }
 
 int cuda_fail(scgpu_ctx* c, cudaError_t e, const char* where) {
+    cudaGetLastError();  // reported here: the next call does not find it again
     return fail(c, SCGPU_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
@@ -490,6 +491,7 @@ int graph_kernel_nodes(cudaGraph_t g) {
 }
 
 int build_graph(scgpu_ctx* c, bool stats, bool reorder, cudaGraphExec_t* out) {
+    if (c->fail_graph.now()) return cuda_fail(c, cudaErrorMemoryAllocation, "step graph (SCGPU_FAIL_GRAPH)");
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c->own, cudaStreamCaptureModeThreadLocal));
     enqueue_any_step(c, stats, reorder, c->own);
@@ -1383,34 +1385,62 @@ int scgpu_track(scgpu_ctx* c, int nsteps, double* stats) {
     if (!c->have_bunch) return fail(c, SCGPU_ERR_STATE, "no bunch on the device");
     CK(cudaSetDevice(c->device));
     const bool want = stats != nullptr;
+    const bool graphs = c->use_graphs && (!c->xfn || c->xcapturable);
+    const long long done = c->steps_done;
     cudaStream_t s = c->stream;
+    auto reorders = [c, done](int k) { return c->reorder_every > 0 && ((done + k) % c->reorder_every) == 0; };
+    auto graph_of = [c, want, reorders](int k) -> cudaGraphExec_t& {
+        return (c->b.nbins > 0 ? c->graphs_bins : c->graphs)[want ? 1 : 0][reorders(k) ? 1 : 0];
+    };
+    auto set_left = [c, s](int left) {
+        return cudaMemcpyAsync(&c->b.st->left, &left, sizeof(int), cudaMemcpyHostToDevice, s);
+    };
     CK(cudaEventRecord(c->ev_t0, s));
-    // the steps of this call hand each other pushed positions; a statistics
-    // record needs them unpushed at the end of every step
-    if (nsteps > 1 && !want)
-        CK(cudaMemcpyAsync(&c->b.st->left, &nsteps, sizeof(int), cudaMemcpyHostToDevice, s));
-    for (int k = 0; k < nsteps; ++k) {
-        const bool reorder = c->reorder_every > 0 && (c->steps_done % c->reorder_every) == 0;
-        if (c->use_graphs && (!c->xfn || c->xcapturable)) {
-            cudaGraphExec_t& gx = (c->b.nbins > 0 ? c->graphs_bins : c->graphs)[want ? 1 : 0][reorder ? 1 : 0];
-            if (!gx) {
-                int rc = build_graph(c, want, reorder, &gx);
-                if (rc) return rc;
+    cudaGetLastError();  // what an earlier call left is not this call's
+    // The steps of this call hand each other pushed positions; a statistics
+    // record needs them unpushed at the end of every step.  A run of steps that
+    // do ends before one whose graph is yet to be built: a build that fails
+    // leaves the bunch after a whole step.  Wherever have_bunch is set, `left`
+    // and `pushed` are 0 between calls.
+    const bool hand_on = nsteps > 1 && !want;
+    int run = 0, at = 0;  // steps of the current run, this one's place in it
+    int rc = SCGPU_OK;
+    for (int k = 0; k < nsteps; ++k, ++at) {
+        if (graphs && !graph_of(k) && (rc = build_graph(c, want, reorders(k), &graph_of(k)))) break;
+        if (hand_on && at == run) {
+            for (run = 1; k + run < nsteps && (!graphs || graph_of(k + run));) ++run;
+            at = 0;
+            if (run > 1) CK(set_left(run));
+        }
+        if (graphs) {
+            const cudaError_t e = c->fail_launch.now() ? cudaErrorMemoryAllocation : cudaGraphLaunch(graph_of(k), s);
+            if (e != cudaSuccess) {
+                rc = cuda_fail(c, e, "cudaGraphLaunch");
+                if (run > 1) set_left(at > 0 ? 1 : 0);
+                if (at == 0 || !hand_on) break;
+                // the step before has pushed the positions: without its graph
+                // this one ends them after a whole step
+            } else {
+                c->kernels_launched += (c->b.nbins > 0 ? c->graph_kernels_bins : c->graph_kernels)[want ? 1 : 0][reorders(k) ? 1 : 0];
             }
-            CK(cudaGraphLaunch(gx, s));
-            c->kernels_launched += (c->b.nbins > 0 ? c->graph_kernels_bins : c->graph_kernels)[want ? 1 : 0][reorder ? 1 : 0];
-        } else {
-            enqueue_any_step(c, want, reorder, s);
+        }
+        if (!graphs || rc) {
+            enqueue_any_step(c, want, reorders(k), s);
             c->kernels_uncounted = true;
         }
         ++c->steps_done;
+        if (rc) break;
         if (want)
             CK(cudaMemcpyAsync(stats + (size_t)k * SCGPU_NSTATS, c->b.st->moments, SCGPU_NSTATS * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
     }
-    CK(cudaEventRecord(c->ev_t1, s));
-    CK(cudaGetLastError());
-    int rc = exchange_status(c);
+    cudaEventRecord(c->ev_t1, s);
+    if (cudaError_t e = cudaGetLastError()) {
+        if (hand_on) c->have_bunch = false;  // steps may be missing: the positions may be pushed
+        return rc ? rc : cuda_fail(c, e, "track");
+    }
+    if (rc) return rc;
+    rc = exchange_status(c);
     if (rc == SCGPU_OK) rc = check_device_err(c);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1);

@@ -3,11 +3,27 @@
 // step together, each held in its own context).
 #pragma once
 
+#include <cstdlib>
 #include <string>
 #include <vector>
 
 #include "scgpu.h"
 #include "sc_internal.h"
+
+namespace sc {
+
+// Fault injection for the tests of the error paths: with the environment
+// variable set to k when the object is created, its k-th call of now() is true
+// (the CUDA call it stands for is then not made and counts as refused).
+struct FailAt {
+    int k = 0;
+    explicit FailAt(const char* env) {
+        if (const char* v = std::getenv(env)) k = std::atoi(v);
+    }
+    bool now() { return k > 0 && --k == 0; }
+};
+
+}  // namespace sc
 
 struct scgpu_ctx {
     int device = 0;
@@ -32,6 +48,8 @@ struct scgpu_ctx {
     long long kernels_launched = 0;   // kernels of the steps scgpu_track launched as graphs
     bool kernels_uncounted = false;   // a step ran outside a graph (host exchange)
     bool use_graphs = true;
+    sc::FailAt fail_graph{"SCGPU_FAIL_GRAPH"};    // builds of the step graphs
+    sc::FailAt fail_launch{"SCGPU_FAIL_LAUNCH"};  // launches of the step graphs
     int reorder_every = 32;   // put the particle arrays in cell order every k steps (0: never)
     long long steps_done = 0; // steps since the last upload
     size_t smem_fft = 0;
