@@ -478,7 +478,8 @@ int scgpu_batch_remove(scgpu_batch* batch, int slot);
 /* the context of an occupied slot (NULL otherwise); owned by the batch */
 scgpu_ctx* scgpu_batch_member(scgpu_batch* batch, int slot);
 int scgpu_batch_size(const scgpu_batch* batch);
-/* every occupied slot advances nsteps ParallelTTracker steps */
+/* every occupied slot advances nsteps ParallelTTracker steps; a round that
+ * breaks off ends after whole steps, as scgpu_track does */
 int scgpu_batch_track(scgpu_batch* batch, int nsteps);
 /* scgpu_batch_track in two halves: launch enqueues the steps and returns, so
  * the host can prepare and scgpu_batch_add further bunches (they join at the

@@ -96,6 +96,7 @@ struct scgpu_batch {
     std::map<int, int> fft_variant;  // transform length -> tile-shape variant
     double last_ms = 0.0;
     int in_flight = 0;  // steps launched and not yet waited for
+    FailAt fail_graph{"SCGPU_FAIL_GRAPH"}, fail_launch{"SCGPU_FAIL_LAUNCH"};
     // Contexts of removed bunches, kept with their device buffers for the
     // next bunch on the same mesh: a serving loop then allocates and frees
     // nothing in steady state (cudaMalloc / cudaFree synchronise the device).
@@ -113,7 +114,10 @@ int bfail(scgpu_batch* b, int code, const std::string& what) {
 #define BCK(call)                                                                                    \
     do {                                                                                             \
         cudaError_t e_ = (call);                                                                     \
-        if (e_ != cudaSuccess) return bfail(b, SCGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                                     \
+            cudaGetLastError(); /* reported here: the next call does not find it again */             \
+            return bfail(b, SCGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
+        }                                                                                            \
     } while (0)
 
 void drop_graphs(scgpu_batch* b) {
@@ -296,6 +300,18 @@ int check_flags(scgpu_batch* b) {
     return SCGPU_OK;
 }
 
+int build_graph(scgpu_batch* b, bool reorder, cudaGraphExec_t* out) {
+    if (b->fail_graph.now()) return bfail(b, SCGPU_ERR_CUDA, "step graph (SCGPU_FAIL_GRAPH)");
+    cudaGraph_t g = nullptr;
+    BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    enqueue_step(b, reorder);
+    BCK(cudaStreamEndCapture(b->stream, &g));
+    const cudaError_t e = cudaGraphInstantiate(out, g, cudaGraphInstantiateFlagUseNodePriority);
+    cudaGraphDestroy(g);
+    BCK(e);
+    return SCGPU_OK;
+}
+
 // Enqueues nsteps batched steps on the batch stream and returns.
 int launch(scgpu_batch* b, int nsteps) {
     BCK(cudaSetDevice(b->device));
@@ -305,32 +321,50 @@ int launch(scgpu_batch* b, int nsteps) {
     }
     b->in_flight = nsteps;
     if (b->members.empty()) return SCGPU_OK;
-    BCK(cudaEventRecord(b->ev_t0, b->stream));
+    const long long done = b->steps;
     const int nm = (int)b->members.size();
-    if (nsteps > 1) k_set_left<<<(nm + 127) / 128, 128, 0, b->stream>>>(b->d_tab, nm, nsteps);
-    for (int k = 0; k < nsteps; ++k) {
-        const bool reorder = b->reorder_every > 0 && (b->steps % b->reorder_every) == 0;
-        cudaGraphExec_t& gx = b->graphs[reorder ? 1 : 0];
-        if (!gx && !b->eager_call) {
-            cudaGraph_t g = nullptr;
-            BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-            enqueue_step(b, reorder);
-            cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-            if (e != cudaSuccess) return bfail(b, SCGPU_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-            e = cudaGraphInstantiate(&gx, g, cudaGraphInstantiateFlagUseNodePriority);
-            cudaGraphDestroy(g);
-            if (e != cudaSuccess) return bfail(b, SCGPU_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
+    auto reorders = [b, done](int k) { return b->reorder_every > 0 && ((done + k) % b->reorder_every) == 0; };
+    auto graph_of = [b, reorders](int k) -> cudaGraphExec_t& { return b->graphs[reorders(k) ? 1 : 0]; };
+    auto set_left = [b, nm](int left) { k_set_left<<<(nm + 127) / 128, 128, 0, b->stream>>>(b->d_tab, nm, left); };
+    BCK(cudaEventRecord(b->ev_t0, b->stream));
+    cudaGetLastError();  // what an earlier call left is not this call's
+    // Runs of steps that hand each other pushed positions, as in scgpu_track:
+    // one ends before a step whose graph is yet to be built
+    const bool hand_on = nsteps > 1;
+    int run = 0, at = 0;
+    int rc = SCGPU_OK;
+    for (int k = 0; k < nsteps; ++k, ++at) {
+        if (!b->eager_call && !graph_of(k) && (rc = build_graph(b, reorders(k), &graph_of(k)))) break;
+        if (hand_on && at == run) {
+            for (run = 1; k + run < nsteps && (b->eager_call || graph_of(k + run));) ++run;
+            at = 0;
+            if (run > 1) set_left(run);
         }
-        if (gx)
-            BCK(cudaGraphLaunch(gx, b->stream));
-        else
-            enqueue_step(b, reorder);
+        const cudaGraphExec_t gx = graph_of(k);
+        if (gx) {
+            const cudaError_t e = b->fail_launch.now() ? cudaErrorMemoryAllocation : cudaGraphLaunch(gx, b->stream);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                rc = bfail(b, SCGPU_ERR_CUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
+                if (run > 1) set_left(at > 0 ? 1 : 0);
+                if (at == 0 || !hand_on) break;
+                // the step before has pushed the positions: without its graph
+                // this one ends them after a whole step
+            }
+        }
+        if (!gx || rc) enqueue_step(b, reorders(k));
         ++b->steps;
+        if (rc) break;
     }
-    BCK(cudaEventRecord(b->ev_t1, b->stream));
-    BCK(cudaGetLastError());
-    b->eager_call = false;
-    return SCGPU_OK;
+    b->in_flight = (int)(b->steps - done);
+    cudaEventRecord(b->ev_t1, b->stream);
+    if (cudaError_t e = cudaGetLastError()) {
+        if (hand_on)  // steps may be missing: the positions may be pushed
+            for (int m : b->members) b->slots[m]->have_bunch = false;
+        return rc ? rc : bfail(b, SCGPU_ERR_CUDA, std::string("batched steps: ") + cudaGetErrorString(e));
+    }
+    if (rc == SCGPU_OK) b->eager_call = false;
+    return rc;
 }
 
 // Waits for the launched steps; device error flags become the status.

@@ -70,3 +70,45 @@ def test_track_that_breaks_off(gpu, kind, failure, monkeypatch):
         c.track(6)
         w.track(6)
         _same(c, w)
+
+
+# whole steps of a round of 20 after one of 1 (the batch reorders at steps 0
+# and 16, the first round after a change of members runs without graphs)
+BATCH_FAILURES = [("SCGPU_FAIL_GRAPH", 1, 0), ("SCGPU_FAIL_GRAPH", 2, 15), ("SCGPU_FAIL_LAUNCH", 1, 0),
+                  ("SCGPU_FAIL_LAUNCH", 2, 2), ("SCGPU_FAIL_LAUNCH", 16, 15), ("SCGPU_FAIL_LAUNCH", 17, 17)]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("failure", BATCH_FAILURES, ids=lambda f: f"{f[0][11:].lower()}{f[1]}")
+def test_batch_round_that_breaks_off(gpu, precision, failure, monkeypatch):
+    def batch(fail):
+        if fail:
+            monkeypatch.setenv(fail[0], str(fail[1]))
+        b = gpu.Batch(precision=precision)
+        if fail:
+            monkeypatch.delenv(fail[0])
+        for i, (n, m) in enumerate([(N, 16), (700, 20)]):
+            R, P = gaussian_bunch(n, bunch_id=i)
+            b.add((m, m, m), R, P, DT, -1e-10 / n, MASS)
+        b.track(1)
+        return b
+
+    def same(b, w):
+        for slot in range(2):
+            _same(b.member(slot), w.member(slot))
+
+    with batch(failure) as b, batch(None) as w:
+        with pytest.raises(gpu.ScgpuError) as e:
+            b.track(20)
+        assert e.value.code == -6
+        b.wait()
+        if failure[2]:
+            w.track(failure[2])
+        same(b, w)
+        for x in (b, w):
+            x.track(1)
+        same(b, w)
+        b.launch(6)
+        b.wait()
+        w.track(6)
+        same(b, w)
