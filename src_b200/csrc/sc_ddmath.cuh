@@ -9,7 +9,9 @@
 // relative accuracy until the last rounding, so they return the correctly
 // rounded result except when the exact value lies within roughly 2^-20 ulp
 // of a rounding boundary; they use only +, -, *, /, sqrt-free fma, and table
-// reads, and give the same bits on the host and on the device.
+// reads (the quick atan also an approximate reciprocal), and log_dd and
+// atan_dd give the same bits on the host and on the device.  atan_fast, which
+// has no rounding test, need not: its reciprocal and its table row may differ.
 //
 // Methods:
 //   * error-free transformations TwoSum (Knuth), Fast2Sum (Dekker) and
@@ -216,6 +218,11 @@ SC_DDM_HD double double_of(uint64_t b) {
     return x;
 }
 
+// Tang's table-driven scheme in the form with short tabulated reciprocals
+// instead of a division (r = z rc - 1 in one fused multiply-add), the exponent
+// and the table row read from the bits of x less those of the first interval's
+// start, as Arm's Optimized Routines (S. Nagy, 2018) publish it; the intervals,
+// reciprocals and tables are our own (gen_ddmath_tables.py).
 // log x = k log 2 - log rc + log1p r for finite normal x: z = x 2^-k in
 // [0.707, 1.414), rc a short reciprocal of z's interval (kLogQ), r = z rc - 1
 // exact, |r| <= 2^-7.  k log 2 (high part) - log rc (high part) is exact
@@ -261,8 +268,9 @@ SC_DDM_HD bool log_quick(double x, double& out) {
     return exact && out == v.hi + (v.lo - kLogQuickErr);
 }
 
-// Reciprocal of d in [1, 2^31] to about 2^-52: an approximation to 2^-20 and
-// one step of third order.
+// Reciprocal of d in [1, 2^31] to 2^-51: an approximation r to 2^-20 and one
+// step r (1 + e + e^2), e = 1 - d r, of Chebyshev's third-order iteration for
+// the zero of 1/x - d.
 SC_DDM_HD double rcp_approx(double d) {
     double r;
 #ifdef __CUDA_ARCH__
@@ -345,8 +353,10 @@ SC_DDM_HD double atan_dd(double x) {
 }
 
 // The same reductions without the rounding test (the mixed form): hi + lo
-// rounded once, within 0.5001 ulp for log and atan of the arguments the
-// quick phases take (log next to 1 within an ulp).
+// rounded once, of the arguments the quick phases take.  By their error bounds
+// within 0.5001 ulp for atan and for log where |log x| >= 2, within 0.513 for
+// log nearer 1 (largest seen: 0.50001, 0.50001 and 0.5055;
+// tests/ddmath_fast_check.cpp).
 SC_DDM_HD double log_fast(double x) {
     if (!log_range(x)) return log(x);
     bool exact;
