@@ -177,7 +177,8 @@ int scgpu_synchronize(scgpu_ctx* ctx);
 int scgpu_compute_potential(scgpu_ctx* ctx, double* rho_inout, const double hr[3]);
 /* the same on a device buffer of the context's GPU (device or managed memory
  * holding nx*ny*nz doubles); anything else returns SCGPU_ERR_ARG before any
- * work is enqueued */
+ * work is enqueued.  The buffer is transformed in place: after SCGPU_ERR_CUDA
+ * its contents are undefined. */
 int scgpu_compute_potential_device(scgpu_ctx* ctx, double* rho_inout_device, const double hr[3]);
 
 /* PartBunch::computeSelfFields on a bunch already in the beam frame: boundp,

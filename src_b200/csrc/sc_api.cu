@@ -759,9 +759,9 @@ static void fork_green(scgpu_ctx* c, bool image, cudaStream_t main) {
 // through the shifted Green's function.  The Green's function is the longer
 // half, so the copy in and passes A, B run beside it, and a device buffer is
 // transformed from and back into in place, which saves two copies (the mixed
-// form converts it first): a solve on the device takes 51 us at 16^3 (60 one
-// after the other, with the copies), 88 at 40 x 20 x 60 (107), 303 at 128^3
-// (330).  A host buffer, managed memory (its pages would move one by one) and
+// form converts it first).  One after the other with the copies -> this: 60 ->
+// 51 us at 16^3, 107 -> 88 at 40 x 20 x 60, 330 -> 303 at 128^3 (265 since the
+// z transforms of 256 points run in registers).  A host buffer, managed memory (its pages would move one by one) and
 // a buffer not aligned to its elements go through the context's grids.
 static int solve_impl(scgpu_ctx* c, double* rho, const double hr[3], bool image, double zshift, bool device_ptr) {
     if (!c || !rho || !hr) return fail(c, SCGPU_ERR_ARG, "null argument");
@@ -1421,7 +1421,8 @@ int scgpu_track(scgpu_ctx* c, int nsteps, double* stats) {
                 // the step before has pushed the positions: without its graph
                 // this one ends them after a whole step
             } else {
-                c->kernels_launched += (c->b.nbins > 0 ? c->graph_kernels_bins : c->graph_kernels)[want ? 1 : 0][reorders(k) ? 1 : 0];
+                auto& nodes = c->b.nbins > 0 ? c->graph_kernels_bins : c->graph_kernels;
+                c->kernels_launched += nodes[want ? 1 : 0][reorders(k) ? 1 : 0];
             }
         }
         if (!graphs || rc) {

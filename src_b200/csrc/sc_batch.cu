@@ -190,10 +190,12 @@ int rebuild(scgpu_batch* b) {
     };
     auto cells = [](const DevBunch& d) { return (long long)d.bc.n[0] * d.bc.n[1] * d.bc.n[2]; };
     const int dep = b->dep_threads;
-    // Particle kernels: as many particles per thread, in every bunch, as fill
-    // the resident blocks once (148 SMs, three blocks of 256), so a block's
-    // set-up and reduction serve several passes; at most 16, so that large
-    // bunches still spread over enough blocks to balance small ones.
+    // Particle kernels: the same number of particles per thread in every
+    // bunch, so a block's set-up and reduction serve several passes: one while
+    // the blocks of 256 do not fill 444 slots (148 SMs, three blocks) twice,
+    // then as many as leave between one and two times the slots; at most 16,
+    // so that large bunches still spread over enough blocks to balance small
+    // ones.
     long long particle_blocks = 0;
     for (const DevBunch& d : tab) particle_blocks += (d.bc.N + 255) / 256;
     const long long per_thread = std::min<long long>(16, std::max<long long>(1, particle_blocks / (148 * 3)));

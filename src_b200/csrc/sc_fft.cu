@@ -21,9 +21,11 @@
 // G on (n0+1)(n1+1)(n2+1) points; it is built here from G with the same FFT
 // stages applied to the even extension of each line.
 //
-// Every kernel stages its lines global -> shared with cp.async (all copies of
-// a block in flight at once, no register round trip), runs Stockham radix
-// stages in shared memory and writes the pruned output.  The transform
+// The staged kernels copy their lines global -> shared with cp.async (all
+// copies of a block in flight at once, no register round trip), run Stockham
+// radix stages in shared memory and write the pruned output; the k_*_lines
+// kernels hold lines of 32 to 256 points in registers (sc_fft_lines.cuh), and
+// sc_fft_plane.cu has the y and x passes of a plane in one kernel.  The transform
 // lengths of the common meshes (2n = 32, 64, 96, 128, 256) are template
 // constants, so the stage loops unroll and the index arithmetic folds; other
 // lengths take the same kernels with the length read at run time.
@@ -1495,7 +1497,8 @@ inline bool special_length(int L) { return L == 32 || L == 64 || L == 96 || L ==
 
 bool fft_register_lines() { return register_lines(); }
 
-// Up to 40^3 cells the step waits on its launches, and the separate assembly
+// Open z, n2 = 16 or 32 (pass A's line kernel of 32 or 64 points) and at most
+// 64000 cells: there the step waits on its launches, and the separate assembly
 // is one (32^3, 1e5 particles: 51.0 -> 48.0 us a step, mixed 47.7 -> 45.5); at
 // 64^3 the assembly fills the GPU and does its divisions faster than the
 // transform's threads between their loads (mixed 107.5 against 109.2 us).

@@ -197,8 +197,8 @@ __global__ void __cluster_dims__(PlaneGeo<L>::CL, 1, 1) __launch_bounds__(PlaneG
 // passes write it to global memory and launch a second kernel).  One block
 // per plane leaves SMs to the deposit that runs beside it.  With the z pass
 // on 256 threads, Green's-function phase 22.4 -> 16.4 us at 16^3, 25.0 -> 19.6
-// at 32^3, unchanged at 64^3 (36 us), where the step gains the launch.  At
-// 256 points a plane and its lines do not fit one block's shared memory.
+// at 32^3, unchanged at 64^3 (36 us; 33.8 since k_dct_z_lines), where the step
+// gains the launch.  At 256 points a plane and its lines do not fit one block's shared memory.
 template <int L>
 struct DctGeo {
     using G = LineGeo<L>;

@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(kThreads) k_assemble_rho(BunchConst bc, const 
 // eight-corner cancellation.
 // CR: the correctly rounded atan / log of the plain form (rounding test,
 // double-double where it cannot decide); otherwise the quick evaluations
-// rounded once (within 0.5001 ulp), the mixed form's Green's function.
+// rounded once (within 0.513 ulp), the mixed form's Green's function.
 template <bool CR = true>
 __device__ __forceinline__ double igf_antiderivative(double x, double y, double z, double cellVolume) {
     double r = sqrt(x * x + y * y + z * z);
@@ -1852,11 +1852,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_gather_kick_push(BunchConst bc,
 }
 constexpr size_t kGatherSmem = kWarps * 2 * 6 * kStreamChunk * sizeof(double);
 template <typename T, bool EXT = false>
-__global__ void __launch_bounds__(kThreads, EXT || sizeof(T) == sizeof(double) ? 3 : 4) k_gather_staged(BunchConst bc, double* __restrict__ x, double* __restrict__ y,
-                                                               double* __restrict__ z, double* __restrict__ px,
-                                                               double* __restrict__ py, double* __restrict__ pz,
-                                                               const T* __restrict__ E4, StepState* st, double* partials,
-                                                               unsigned* ticket) {
+__global__ void __launch_bounds__(kThreads, EXT || sizeof(T) == sizeof(double) ? 3 : 4)
+    k_gather_staged(BunchConst bc, double* __restrict__ x, double* __restrict__ y, double* __restrict__ z,
+                    double* __restrict__ px, double* __restrict__ py, double* __restrict__ pz, const T* __restrict__ E4,
+                    StepState* st, double* partials, unsigned* ticket) {
     extern __shared__ __align__(16) double gather_sm[];
     gather_body<T, false, EXT, true>(bc, x, y, z, px, py, pz, E4, st, partials, ticket, vb_grid(), nullptr, gather_sm);
 }
@@ -2201,7 +2200,8 @@ int wave_grid(K kernel, const DevBunch& b, size_t smem = 0) {
 }
 
 // The gather streams the particle state through shared memory with bulk
-// copies (default); SCGPU_STREAM=0 selects the direct-load kernel (same bits).
+// copies (default); SCGPU_STREAM=0 selects the direct-load kernel (same bits;
+// single bunches only, a batch always streams).
 bool stream_particles() {
     static const bool on = [] {
         const char* e = std::getenv("SCGPU_STREAM");
